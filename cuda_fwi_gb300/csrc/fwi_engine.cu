@@ -30,6 +30,7 @@
 #include "fwi_kernels.cuh"
 #include "fwi_tma.cuh"
 #include "fwi_fused.cuh"
+#include "fwi_resident.h"
 
 namespace fwi {
 
@@ -649,11 +650,15 @@ static size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 // kernel recorded since the last call, reported and cleared.
 static int check_bounds_record() {
 #if FWI_BOUNDS_CHECK
-    unsigned long long v = 0;
+    unsigned long long v = 0, w = 0;
     CUDA_TRY(cudaMemcpyFromSymbol(&v, g_fwi_oob, sizeof(v)));
+    CUDA_TRY(resident_bounds_record(&w));
     if (v) {
         const unsigned long long zero = 0;
         CUDA_TRY(cudaMemcpyToSymbol(g_fwi_oob, &zero, sizeof(zero)));
+    }
+    if (!v) v = w;
+    if (v) {
         return fail(FWI_ERR_CUDA, "out-of-range index " + std::to_string((long long)(v & 0xFFFFFFFFFFFFull)) +
                                       " at access site " + std::to_string((int)(v >> 48)) + "; results discarded");
     }
@@ -753,6 +758,20 @@ struct Engine {
     std::vector<FusedMaps> fmaps_b;
     FusedGrid fgrid{};
     int grid_fused = 1;
+    // Resident time loops (fwi_resident.cuh): kernels of the half order, the
+    // tiling of the current batch's forward and backward (shots 0: not used),
+    // inboxes, programs and per-tile events
+    struct ResPlan {
+        int shots = 0;  // shots per launch
+        ResTiling t{};
+        int mode = RES_FORWARD;
+    };
+    ResSet rset{};
+    ResPlan res_f, res_b;
+    DBuf d_inbox, d_rops_f, d_rops_b, d_revo_f, d_rev_f, d_revo_a, d_rev_a;
+    std::string rops_key_f, rops_key_b;  // what the programs on the device were made for
+    int nrops_f = 0, nrops_b = 0;
+    unsigned res_tag = 0;  // last exchange tag used
     unsigned long long wait_ns = kWaitNs;  // limit of the kernels' bounded waits
     bool stall_next = false, stall_pending = false;  // test hook: one forward step whose wait runs out
     bool zero_mu = false;  // some interior cell has mu == 0 (exact mode unsupported)
@@ -851,6 +870,11 @@ struct Engine {
         xs = exact_for(fpad);
         tset = tma_for(fpad);
         fset = fused_for(fpad);
+        rset = resident_for(fpad);
+        int coop = 0;
+        CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+        if (coop) CUDA_TRY(rset.prepare());
+        else rset.launch = nullptr;
         if (kmap == 3) CUDA_TRY(tset.prepare());
         if (kmap == 3 && fset.prepare) CUDA_TRY(fset.prepare());
         CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
@@ -1100,6 +1124,10 @@ struct Engine {
         return FWI_OK;
     }
 
+    // one injection or recording of a batch slot
+    struct Ev {
+        int x, z, kind, idx, code;
+    };
     int setup_batch(int nb, const int* ids, bool keep) {
         if (!have_model) return fail(FWI_ERR_STATE, "set a model first");
         if (nb < 1 || !ids) return fail(FWI_ERR_INVALID, "empty shot batch");
@@ -1185,7 +1213,7 @@ struct Engine {
         fwd_kept = false;
         bwd_done = false;
         // events per slot, grouped by column, sorted by (z, inject-before-record, index)
-        struct Ev { int x, z, kind, idx, code; };
+        std::vector<std::vector<Ev>> slot_f(B), slot_a(B);
         std::vector<int> colf((size_t)B * (nxt + 1)), cola((size_t)B * (nxt + 1));
         std::vector<int2> evf, eva;
         std::vector<int> evxf, evxa;
@@ -1222,6 +1250,8 @@ struct Engine {
             };
             fill(ef, colf, evf, evxf);
             fill(ea, cola, eva, evxa);
+            slot_f[b].swap(ef);
+            slot_a[b].swap(ea);
         }
         // event tables are reached through the item descriptors only (not captured)
         FWI_TRY(d_evcol_f.ensure(colf.size() * 4));
@@ -1279,9 +1309,257 @@ struct Engine {
         }
         FWI_TRY(tiles_for(B));
         if (kmap == 3) FWI_TRY(build_tma_maps());
-        CUDA_TRY(cudaStreamSynchronize(stream));
         if (keep && ckpt_mode()) plan = plan_binomial(nunits(), slots, &plan_cost);
+        res_f = resident_plan(RES_FORWARD);
+        res_b = keep ? resident_plan(ckpt_mode() ? RES_BOTH : RES_STORED) : ResPlan{};
+        if (res_f.shots) FWI_TRY(resident_events(res_f, slot_f, d_revo_f, d_rev_f));
+        if (res_b.shots) {
+            if (res_b.mode == RES_BOTH) FWI_TRY(resident_events(res_b, slot_f, d_revo_a, d_rev_a, &slot_a));
+            else FWI_TRY(resident_events(res_b, slot_a, d_revo_a, d_rev_a));
+        }
+        CUDA_TRY(cudaStreamSynchronize(stream));
         return FWI_OK;
+    }
+
+    // ---- resident time loops --------------------------------------------------
+    // Tiling of the batch for the resident kernels (shots per launch and tiles per
+    // shot), or shots = 0 where the launches per pass are expected to be faster or
+    // the fields do not fit in shared memory.
+    //
+    // The expectation, in us per time step, fitted to both schedules on grids of
+    // 0.06 to 1 M cells (orders 2..12, CPML 0..30): a resident step is two halo
+    // exchanges (~1.1 us each) and, per row that a thread marches through, the
+    // stencils of both passes (kRowUs by half order; above 4 the windows spill);
+    // a step of launches is ~12 us of launch and pipeline latency and 14 us per
+    // M cells.  Measured, resident / launches: 200x200 order 4 3.1 / 12.1, order 8
+    // 3.9 / 12.7, 600x380 order 8 5.7 / 16.3, 800x400 order 8 8.7 / 20.0, 403x307
+    // order 12 two shots 16 / 20, six shots (three launches) 48 / 27.  A
+    // checkpointed backward adds, per adjoint step, the gradient's and ux/uz's
+    // round trips to L2 and about two saves and restores of the state.
+    ResPlan resident_plan(int mode) const {
+        ResPlan best;
+        if (bx_req != 0 || tz_req != 0 || kmap != 3 || fuse || exact() || random_mode() || snap_interval > 0 ||
+            !rset.launch)
+            return best;
+        static constexpr double kRowUs[kMaxHalf] = {1.2, 1.2, 1.7, 1.8, 3.3, 3.8};
+        const int pairs = res_pairs(nxt, fpad), nz = nzt - 2 * fpad, most = kResTX / 2;
+        const int min_rows = fsurf ? fpad + 1 : fpad;
+        const double mcells = 1e-6 * B * (double)(nxt - 2 * fpad) * nz;
+        const double again = mode == RES_BOTH ? (double)plan_recompute() / std::max(nunits(), 1) : 0.0;
+        const double pass_us = 11.5 + 14.0 * mcells;
+        double best_us = mode == RES_BOTH ? again * pass_us + 9.5 + 19.0 * mcells : pass_us;
+        for (int k = 1; k <= std::min(B, num_sms); k++) {
+            const int launches = (B + k - 1) / k;
+            if (k > 1 && (B + k - 2) / (k - 1) == launches) continue;  // no fewer launches than k - 1
+            const int tiles = num_sms / k;
+            for (int ntx = (pairs + most - 1) / most; ntx <= tiles && 2 * (pairs / ntx) >= 16; ntx++) {
+                const int ntz = std::min(tiles / ntx, nz / min_rows);
+                if (ntz < 1) break;
+                ResTiling t{ntx, ntz, (nz + ntz - 1) / ntz, 0, 0};
+                strips_of(t);
+                if (t.tzm > kResThreads / 4 || rset.smem(t, tp, mode) > (size_t)kResSmem) continue;
+                const int npm = (pairs + ntx - 1) / ntx, gw = npm > 16 ? 32 : npm > 8 ? 16 : 8;
+                const int groups = std::min(t.tzm, kResThreads / gw), rows_each = (t.tzm + groups - 1) / groups;
+                // (a tie goes to the smaller perimeter)
+                const double step_us = 2.2 + rows_each * kRowUs[fpad - 1] + 0.002 * (t.tzm + npm);
+                const double us = launches * (mode == RES_BOTH ? again * step_us + 2.0 + 10.5 * rows_each : step_us);
+                if (us < best_us) {
+                    best_us = us;
+                    best.shots = k;
+                    best.t = t;
+                    best.mode = mode;
+                }
+            }
+        }
+        return best;
+    }
+    // Room for the CPML strips of a tiling's tiles.
+    void strips_of(ResTiling& t) const {
+        const int pairs = res_pairs(nxt, fpad), nz = nzt - 2 * fpad;
+        const ResStrips st = res_strips(nzt, nxt, ppad, npml, fsurf);
+        for (int i = 0; i < t.ntx; i++) {
+            const int p0 = res_cut(pairs, t.ntx, i), np = res_cut(pairs, t.ntx, i + 1) - p0;
+            const int x0 = res_xb(fpad) + 2 * p0;
+            const int nl = std::min(std::max((st.left - x0 + 1) / 2, 0), np);
+            const int fr = std::min(std::max((st.right - x0) / 2, 0), np);
+            if (npml > 0) t.sxp = std::max(t.sxp, nl + np - fr);
+        }
+        for (int i = 0; i < t.ntz; i++) {
+            const int z0 = fpad + res_cut(nz, t.ntz, i), nr = res_cut(nz, t.ntz, i + 1) - (z0 - fpad);
+            const int top = std::min(std::max(st.top - z0, 0), nr), bot = std::min(std::max(st.bottom - z0, 0), nr);
+            if (npml > 0) t.szr = std::max(t.szr, top + nr - bot);
+        }
+    }
+    // Events of every tile of the batch: offsets [B * tiles + 1] and (cell, code)
+    // in event order.  With `second`, its lists follow those of `first` (offsets
+    // of both, B * tiles + 1 each, in one array).
+    int resident_events(const ResPlan& rp, const std::vector<std::vector<Ev>>& first, DBuf& off, DBuf& ev,
+                        const std::vector<std::vector<Ev>>* second = nullptr) {
+        const int per = rp.t.ntx * rp.t.ntz;
+        const int xb = res_xb(fpad), pairs = res_pairs(nxt, fpad), nz = nzt - 2 * fpad;
+        std::vector<int> tx_of(pairs), tz_of(nz);
+        for (int t = 0; t < rp.t.ntx; t++)
+            for (int p = res_cut(pairs, rp.t.ntx, t); p < res_cut(pairs, rp.t.ntx, t + 1); p++) tx_of[p] = t;
+        for (int t = 0; t < rp.t.ntz; t++)
+            for (int r = res_cut(nz, rp.t.ntz, t); r < res_cut(nz, rp.t.ntz, t + 1); r++) tz_of[r] = t;
+        std::vector<int> o;
+        std::vector<int2> e;
+        for (const auto* lists : {&first, second}) {
+            if (!lists) continue;
+            std::vector<std::vector<int2>> tile((size_t)B * per);
+            for (int b = 0; b < B; b++)
+                for (const Ev& v : (*lists)[b]) {
+                    const int tx = tx_of[(v.x - xb) / 2], tz = tz_of[v.z - fpad];
+                    const int x0 = xb + 2 * res_cut(pairs, rp.t.ntx, tx), z0 = fpad + res_cut(nz, rp.t.ntz, tz);
+                    auto& list = tile[(size_t)b * per + tz * rp.t.ntx + tx];
+                    const int cell = (v.z - z0) * rset.pitch + v.x - x0;
+                    const bool more = !list.empty() && (list.back().x & (kResMore - 1)) == cell;
+                    list.push_back(make_int2(cell | (more ? kResMore : 0), v.code));
+                }
+            for (const auto& t : tile) {
+                o.push_back((int)e.size());
+                e.insert(e.end(), t.begin(), t.end());
+            }
+            o.push_back((int)e.size());
+        }
+        FWI_TRY(off.ensure(o.size() * 4));
+        FWI_TRY(ev.ensure(std::max<size_t>(1, e.size()) * 8));
+        CUDA_TRY(cudaMemcpyAsync(off.p, o.data(), o.size() * 4, cudaMemcpyHostToDevice, stream));
+        if (!e.empty()) CUDA_TRY(cudaMemcpyAsync(ev.p, e.data(), e.size() * 8, cudaMemcpyHostToDevice, stream));
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        return FWI_OK;
+    }
+    int resident_program(const std::vector<ResOp>& ops, DBuf& buf, int* n) {
+        FWI_TRY(buf.ensure(ops.size() * sizeof(ResOp)));
+        CUDA_TRY(cudaMemcpyAsync(buf.p, ops.data(), ops.size() * sizeof(ResOp), cudaMemcpyHostToDevice, stream));
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        *n = (int)ops.size();
+        return FWI_OK;
+    }
+    // The program of a forward sweep (recording; saves: state, slot) or of a
+    // backward, for every shot of the batch.  `passes` bounds the exchange tags used.
+    int resident_run(const ResPlan rp, const DBuf& ops, int nops, bool backward, long long passes) {
+        const int per = rp.t.ntx * rp.t.ntz;
+        const size_t words = (size_t)rset.inbox_words(rp.t.tzm);
+        const size_t bytes = (size_t)rp.shots * per * 4 * words * 8, before = d_inbox.bytes;
+        FWI_TRY(d_inbox.ensure(bytes));
+        ResArgs a{};
+        a.t = rp.t;
+        a.nops = nops;
+        a.ops = ops.as<ResOp>();
+        a.inbox = d_inbox.as<unsigned long long>();
+        a.slot_stride = (long long)B * state;
+        a.state = (long long)state;
+        a.field = (long long)field;
+        a.xstrip = (long long)xstrip;
+        a.zstrip = (long long)zstrip;
+        a.nf = (long long)nf;
+        a.nft = nft;
+        a.err = d_err.as<int>();
+        a.wait_ns = wait_ns ? wait_ns : kWaitNs;
+        a.one = 1.f;
+        for (int b = 0; b < B; b += rp.shots) {
+            const int n = std::min(rp.shots, B - b);
+            // tags only grow (words of earlier launches never match); fresh memory
+            // and a counter about to wrap start over from zeroed words
+            if (d_inbox.bytes != before || passes > (long long)(0xFFFFFFF0u - res_tag)) {
+                if (b == 0 || passes > (long long)(0xFFFFFFF0u - res_tag)) {
+                    CUDA_TRY(cudaMemsetAsync(d_inbox.p, 0, d_inbox.bytes, stream));
+                    res_tag = 0;
+                }
+            }
+            a.tag0 = res_tag;
+            res_tag += (unsigned)passes;
+            fill_item(a.f, b, false);
+            fill_item(a.a, b, true);
+            a.snap = d_snap.p ? d_snap.as<float>() + (size_t)b * state : nullptr;
+            const int* off = (backward ? d_revo_a : d_revo_f).as<int>() + (size_t)b * per;
+            const int2* ev = (backward ? d_rev_a : d_rev_f).as<int2>();
+            a.evo_f = off;
+            a.ev_f = ev;
+            a.evo_a = rp.mode == RES_BOTH ? off + (size_t)B * per + 1 : off;
+            a.ev_a = ev;
+            const cudaError_t ce = rset.launch(rp.mode, n * per, stream, a);
+            if (ce == cudaErrorCooperativeLaunchTooLarge) {
+                // this context has fewer SMs than the device (before any launch ran: the
+                // first is the largest): the launches per pass do it
+                cudaGetLastError();
+                rset.launch = nullptr;
+                res_f = res_b = ResPlan{};
+                return FWI_OK;
+            }
+            CUDA_TRY(ce);
+            launches_now++;
+        }
+        return FWI_OK;
+    }
+    int resident_forward(const std::vector<std::pair<int, int>>& saves, bool store) {
+        const std::string key = "f" + shape_key() + (store ? "S" : "") + "|sv" + std::to_string(saves.size());
+        if (key != rops_key_f) {
+            std::vector<ResOp> ops;
+            const int fl = (int)(FL_WE | FL_RECORD | (store ? FL_STORE : 0u));
+            int t = 0;
+            for (const auto& sv : saves) {
+                const int ts = sv.first * unit();
+                ops.push_back({RES_ADV, t, ts, fl});
+                ops.push_back({RES_SAVE, sv.second, 0, 0});
+                t = ts;
+            }
+            ops.push_back({RES_ADV, t, nt, fl});
+            ops.push_back({RES_FINAL, 0, 0, 0});
+            rops_key_f.clear();
+            FWI_TRY(resident_program(ops, d_rops_f, &nrops_f));
+            rops_key_f = key;
+        }
+        CUDA_TRY(cudaMemsetAsync(d_fwd.p, 0, (size_t)B * state * 4, stream));
+        CUDA_TRY(cudaMemsetAsync(d_ws.p, 0, (size_t)B * field * 4, stream));
+        FWI_TRY(resident_run(res_f, d_rops_f, nrops_f, false, (long long)nt + 1));
+        if (res_f.shots && !rows.empty()) {
+            const int blocks = (int)std::min<size_t>((rows.size() * nt + 255) / 256, (size_t)num_sms * 4);
+            watch_traces_kernel<<<std::max(blocks, 1), 256, 0, stream>>>(d_rec.as<float>(), (int)rows.size(), nt, 0, nt,
+                                                                         d_err.as<int>());
+            launches_now++;
+        }
+        return FWI_OK;
+    }
+    int resident_backward() {
+        const std::string key = "b" + shape_key();
+        const int gf = grad_on ? (int)FL_GRAD : 0;
+        if (key != rops_key_b) {
+            std::vector<ResOp> ops;
+            if (!ckpt_mode()) {
+                ops.push_back({RES_ADJ, 0, nt, gf | (int)FL_WE});
+            } else {
+                size_t k = 0;
+                int last_slot = -1, last_state = 0;
+                while (k < plan.size() && plan[k].kind != Action::ADJOINT) {
+                    if (plan[k].kind == Action::SAVE) { last_slot = plan[k].a; last_state = plan[k].b; }
+                    k++;
+                }
+                const int u = unit();
+                ops.push_back({RES_RESTORE, last_slot, 0, 0});
+                ops.push_back({RES_ADV, last_state * u, (nunits() - 1) * u, 0});
+                for (; k < plan.size(); k++) {
+                    const Action& a = plan[k];
+                    if (a.kind == Action::ADVANCE) ops.push_back({RES_ADV, a.a * u, a.b * u, 0});
+                    else if (a.kind == Action::SAVE) ops.push_back({RES_SAVE, a.a, 0, 0});
+                    else if (a.kind == Action::RESTORE) ops.push_back({RES_RESTORE, a.a, 0, 0});
+                    else ops.push_back({RES_ADJ, a.a * u, std::min(nt, (a.a + 1) * u), gf | (int)FL_WE});
+                }
+            }
+            ops.push_back({RES_FINAL, 1, 0, 0});
+            rops_key_b.clear();
+            FWI_TRY(resident_program(ops, d_rops_b, &nrops_b));
+            rops_key_b = key;
+        }
+        CUDA_TRY(cudaMemsetAsync(d_adj.p, 0, (size_t)B * state * 4, stream));
+        CUDA_TRY(cudaMemsetAsync(d_wr.p, 0, (size_t)B * field * 4, stream));
+        CUDA_TRY(cudaMemsetAsync(d_ux.p, 0, (size_t)B * field * 4, stream));
+        CUDA_TRY(cudaMemsetAsync(d_uz.p, 0, (size_t)B * field * 4, stream));
+        CUDA_TRY(cudaMemsetAsync(d_grad.p, 0, (size_t)B * 3 * nf * 4, stream));
+        // a restored state publishes its halos too
+        return resident_run(res_b, d_rops_b, nrops_b, true,
+                            (long long)nt + nrops_b + (ckpt_mode() ? plan_recompute() * unit() : 0) + 1);
     }
     // Maps of the fused step, per buffer it can read from.
     int build_fused_maps() {
@@ -1793,7 +2071,8 @@ struct Engine {
         stall_next = false;
         const std::string key = std::string("fwd") + (store ? "S" : "") + (ckpt ? "C" : "") +
                                 (obs ? "O" : "") + (stall_pending ? "X" : "") + shape_key();
-        FWI_TRY(run_phase(key, [&]() -> int {
+        const bool resident_loop = res_f.shots > 0 && !stall_pending;
+        auto sweep = [&]() -> int {
             CUDA_TRY(cudaMemsetAsync(d_fwd.p, 0, (size_t)B * state * 4, stream));
             CUDA_TRY(cudaMemsetAsync(d_ws.p, 0, (size_t)B * field * 4, stream));
             int t = 0;
@@ -1829,6 +2108,9 @@ struct Engine {
                     launches_now += 2;
                 }
             }
+            return FWI_OK;
+        };
+        auto residual = [&]() -> int {
             if (obs && nrows) {
                 CUDA_TRY(cudaMemsetAsync(d_blow.p, 0, 4, stream));
                 residual_kernel<<<(unsigned)nrows, 256, 0, stream>>>(
@@ -1837,7 +2119,16 @@ struct Engine {
                 launches_now++;
             }
             return FWI_OK;
-        }));
+        };
+        if (resident_loop) FWI_TRY(resident_forward(saves, store));
+        if (resident_loop && res_f.shots) {
+            FWI_TRY(residual());
+        } else {
+            FWI_TRY(run_phase(key, [&]() -> int {
+                FWI_TRY(sweep());
+                return residual();
+            }));
+        }
         CUDA_TRY(cudaEventRecord(e1, stream));
         FWI_TRY(h_rec.ensure(rec_out ? nrows * nt * 4 : 16));
         float* rec = h_rec.as<float>();
@@ -1939,7 +2230,8 @@ struct Engine {
         long long recompute = 0;
         CUDA_TRY(cudaEventRecord(e0, stream));
         const std::string key = std::string(ckpt_mode() ? "bwdC" : random_mode() ? "bwdR" : "bwdS") + shape_key();
-        FWI_TRY(run_phase(key, [&]() -> int {
+        if (res_b.shots) FWI_TRY(resident_backward());
+        if (!res_b.shots) FWI_TRY(run_phase(key, [&]() -> int {
             CUDA_TRY(cudaMemsetAsync(d_adj.p, 0, (size_t)B * state * 4, stream));
             CUDA_TRY(cudaMemsetAsync(d_wr.p, 0, (size_t)B * field * 4, stream));
             CUDA_TRY(cudaMemsetAsync(d_ux.p, 0, (size_t)B * field * 4, stream));

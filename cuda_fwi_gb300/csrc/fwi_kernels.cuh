@@ -97,7 +97,7 @@ struct Cpml {
 // the record after each call (FWI_ERR_CUDA "out-of-range index").  Sites of
 // the TMA-staged kernels: 1-2 x-strip CPML of a pair, 11-14 forward stress
 // pass, 21-24 forward velocity pass, 31-36 adjoint stress pass, 41-49 fused
-// forward step.  The cell mappings and the exact adjoint are not guarded.
+// forward step, 51-63 resident time loops.  The cell mappings and the exact adjoint are not guarded.
 #ifndef FWI_BOUNDS_CHECK
 #define FWI_BOUNDS_CHECK 0
 #endif
