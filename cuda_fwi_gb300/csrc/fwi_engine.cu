@@ -109,6 +109,23 @@ __global__ void watch_array_kernel(const float* __restrict__ a, size_t n, int* _
 }
 constexpr int kWatchSteps = 64;  // recorded steps between two watchdog checks
 
+// Event map of one slot (the velocity pass of the TMA mapping reads it): its
+// events lie at [first, end) of the flat tables (columns, (row, code)), sorted by
+// cell; rows ez0.. of `pitch` entries at map.
+static void fill_event_map(int* map, int ez0, int pitch, const std::vector<int>& col, const std::vector<int2>& ev,
+                           size_t first, size_t end) {
+    for (size_t i = first; i < end;) {
+        size_t j = i + 1;
+        while (j < end && col[j] == col[i] && ev[j].x == ev[i].x) j++;
+        const int code = ev[i].y;
+        map[(size_t)(ev[i].x - ez0) * pitch + col[i]] =
+            (int)(j > i + 1 ? EV_LIST | (unsigned)i : code >= 0 ? EV_INJECT | (unsigned)code : EV_RECORD | (unsigned)~code);
+        i = j;
+    }
+}
+// Largest event map that is built (entries): above, events run in their own kernel.
+constexpr size_t kEventMapMax = 512 * 1024;
+
 // Source injection and receiver recording of one batch slot per block, after
 // a velocity pass that did neither (the TMA mapping): the injections of a
 // cell are added in event order by one thread (events are sorted by column,
@@ -729,6 +746,9 @@ struct Engine {
     DBuf d_fwd, d_adj, d_ws, d_wr, d_ux, d_uz, d_grad, d_gsum, d_store, d_snap;
     DBuf d_evcol_f, d_ev_f, d_evcol_a, d_ev_a, d_evx_f, d_evx_a, d_rec, d_resid, d_rowmis, d_blow;
     DBuf d_items_f, d_items_a;
+    DBuf d_evmap_f, d_evmap_a;  // event maps of the batch (rows ez0..ez1 of every slot)
+    int ez0_f = 0, ez1_f = -1, ez0_a = 0, ez1_a = -1;
+    bool ev_map = false;        // the velocity passes inject and record
     // exact discrete adjoint: forward state n+1, derivative adjoints + sensitivities, descriptors
     DBuf d_nxt, d_exact, d_exd, d_items_n;
     ExactSet xs{};
@@ -1253,6 +1273,34 @@ struct Engine {
             slot_f[b].swap(ef);
             slot_a[b].swap(ea);
         }
+        // event maps: the rows with events, the same for every slot of the batch
+        auto rows_of = [](const std::vector<int2>& ev, int* z0, int* z1) {
+            *z0 = 0;
+            *z1 = -1;
+            for (const int2& e : ev) {
+                *z0 = *z1 < *z0 ? e.x : std::min(*z0, e.x);
+                *z1 = std::max(*z1, e.x);
+            }
+        };
+        rows_of(evf, &ez0_f, &ez1_f);
+        rows_of(eva, &ez0_a, &ez1_a);
+        const size_t map_f = (size_t)(ez1_f - ez0_f + 1) * pitch, map_a = (size_t)(ez1_a - ez0_a + 1) * pitch;
+        ev_map = kmap == 3 && B * std::max(map_f, map_a) <= kEventMapMax;
+        if (ev_map) {
+            std::vector<int> mf(B * map_f, 0), ma(B * map_a, 0);
+            for (int b = 0; b < B; b++) {
+                const int *cf = colf.data() + (size_t)b * (nxt + 1), *ca = cola.data() + (size_t)b * (nxt + 1);
+                fill_event_map(mf.data() + b * map_f, ez0_f, pitch, evxf, evf, cf[0], cf[nxt]);
+                fill_event_map(ma.data() + b * map_a, ez0_a, pitch, evxa, eva, ca[0], ca[nxt]);
+            }
+            FWI_TRY(d_evmap_f.ensure(std::max<size_t>(1, mf.size()) * 4));
+            FWI_TRY(d_evmap_a.ensure(std::max<size_t>(1, ma.size()) * 4));
+            if (!mf.empty()) CUDA_TRY(cudaMemcpyAsync(d_evmap_f.p, mf.data(), mf.size() * 4, cudaMemcpyHostToDevice, stream));
+            if (!ma.empty()) CUDA_TRY(cudaMemcpyAsync(d_evmap_a.p, ma.data(), ma.size() * 4, cudaMemcpyHostToDevice, stream));
+        } else {
+            ez0_f = ez0_a = 0;
+            ez1_f = ez1_a = -1;
+        }
         // event tables are reached through the item descriptors only (not captured)
         FWI_TRY(d_evcol_f.ensure(colf.size() * 4));
         FWI_TRY(d_evcol_a.ensure(cola.size() * 4));
@@ -1330,10 +1378,11 @@ struct Engine {
     // 0.06 to 1 M cells (orders 2..12, CPML 0..30): a resident step is two halo
     // exchanges (~1.1 us each) and, per row that a thread marches through, the
     // stencils of both passes (kRowUs by half order; above 4 the windows spill);
-    // a step of launches is ~12 us of launch and pipeline latency and 14 us per
-    // M cells.  Measured, resident / launches: 200x200 order 4 3.1 / 12.1, order 8
-    // 3.9 / 12.7, 600x380 order 8 5.7 / 16.3, 800x400 order 8 8.7 / 20.0, 403x307
-    // order 12 two shots 16 / 20, six shots (three launches) 48 / 27.  A
+    // a step of launches is ~9.5 us of launch and pipeline latency and 14 us per
+    // M cells.  Measured, resident / launches: 200x200 order 4 3.1 / 9.5, order 8
+    // 3.9 / 10.5, 600x380 order 8 5.7 / 13.7, order 12 9.4 / 14.6; 403x307 order 12
+    // six shots (three launches) 48 / 24; checkpointed backward of 200x200 order 4
+    // 16.4 / 28.9, 400x300 order 8 34.2 / 30.4.  A
     // checkpointed backward adds, per adjoint step, the gradient's and ux/uz's
     // round trips to L2 and about two saves and restores of the state.
     ResPlan resident_plan(int mode) const {
@@ -1346,8 +1395,8 @@ struct Engine {
         const int min_rows = fsurf ? fpad + 1 : fpad;
         const double mcells = 1e-6 * B * (double)(nxt - 2 * fpad) * nz;
         const double again = mode == RES_BOTH ? (double)plan_recompute() / std::max(nunits(), 1) : 0.0;
-        const double pass_us = 11.5 + 14.0 * mcells;
-        double best_us = mode == RES_BOTH ? again * pass_us + 9.5 + 19.0 * mcells : pass_us;
+        const double pass_us = 8.8 + 0.25 * fpad + 14.0 * mcells;
+        double best_us = mode == RES_BOTH ? again * pass_us + 8.0 + 22.0 * mcells : pass_us;
         for (int k = 1; k <= std::min(B, num_sms); k++) {
             const int launches = (B + k - 1) / k;
             if (k > 1 && (B + k - 2) / (k - 1) == launches) continue;  // no fewer launches than k - 1
@@ -1774,9 +1823,9 @@ struct Engine {
     }
     void pass_velocity(int w, const ItemDesc* items, int it, unsigned flags) {
         if (kmap == 3) {
+            tset.velocity(dim3(grid_tma), stream, vmaps[w], items, tgrid, it, flags, d_err.as<int>());
             const unsigned ev = flags & (FL_INJECT | FL_RECORD);
-            tset.velocity(dim3(grid_tma), stream, vmaps[w], items, tgrid, it, flags & ~ev, d_err.as<int>());
-            if (ev) {
+            if (ev && !ev_map) {
                 events_kernel<<<B, 256, 0, stream>>>(items, it, ev);
                 launches_now++;
             }
@@ -1789,7 +1838,7 @@ struct Engine {
         return "|B" + std::to_string(B) + "|r" + std::to_string(rows.size()) + "|s" +
                std::to_string(slots) + "|st" + std::to_string(strategy) + "|t" + std::to_string(ntiles) +
                "|g" + std::to_string(grad_on ? 1 : 0) + "|m" + std::to_string(grad_mode) + "|rb" +
-               std::to_string(rb_active ? 1 : 0) + "|fu" + std::to_string(fused() ? 1 : 0) + "|sn" +
+               std::to_string(rb_active ? 1 : 0) + "|em" + std::to_string(ev_map ? 1 : 0) + "|fu" + std::to_string(fused() ? 1 : 0) + "|sn" +
                std::to_string(snap_interval) + "." + std::to_string(snap_field);
     }
 
@@ -1855,6 +1904,9 @@ struct Engine {
         d.ev_col = (adj ? d_evcol_a.as<int>() : d_evcol_f.as<int>()) + (size_t)b * (nxt + 1);
         d.ev = adj ? d_ev_a.as<int2>() : d_ev_f.as<int2>();
         d.ev_x = adj ? d_evx_a.as<int>() : d_evx_f.as<int>();
+        d.ez0 = adj ? ez0_a : ez0_f;
+        d.ez1 = adj ? ez1_a : ez1_f;
+        d.evmap = (adj ? d_evmap_a : d_evmap_f).as<int>() + (size_t)b * std::max(d.ez1 - d.ez0 + 1, 0) * pitch;
         d.inj = adj ? d_resid.as<float>() : d_srcsig.as<float>();
         d.rec = d_rec.as<float>();
         d.store = d_store.p ? d_store.as<float>() + (size_t)b * nft * 5 * nf : nullptr;
@@ -2002,9 +2054,12 @@ struct Engine {
         vm.sxx = vmaps_b[y].sxx;
         vm.szx = vmaps_b[y].szx;
         vm.szz = vmaps_b[y].szz;
-        tset.velocity(dim3(grid_tma), stream, vm, items, gg, it, 0u, d_err.as<int>());
-        events_kernel<<<B, 256, 0, stream>>>(items, it, FL_INJECT);
-        launches_now += 3;
+        tset.velocity(dim3(grid_tma), stream, vm, items, gg, it, FL_INJECT, d_err.as<int>());
+        launches_now += 2;
+        if (!ev_map) {
+            events_kernel<<<B, 256, 0, stream>>>(items, it, FL_INJECT);
+            launches_now++;
+        }
     }
 
     // Run `body` directly or as a cached CUDA graph.

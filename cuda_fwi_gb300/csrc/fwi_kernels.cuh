@@ -60,7 +60,7 @@ struct __align__(16) ItemDesc {
     int pnz, fsurf, nt, fwi_dt;
     int fwi_dx, fwi_dz, wx1, wx2;
     int wz1, wz2, nfz, nfx;
-    int fwd_kind, fwd_xs, pad0, pad1;  // fwd_kind: 0 = storage, 1 = forward state
+    int fwd_kind, fwd_xs, ez0, ez1;  // fwd_kind: 0 = storage, 1 = forward state; evmap rows (none: ez1 < ez0)
     long long fwd_fs, fwd_zs;
     float dt, inv_dt, gscale, pad2;    // gscale = fwi_dt * dt
     float hx[kMaxHalf], hz[kMaxHalf];  // dxi*hc[k], dzi*hc[k]
@@ -78,11 +78,18 @@ struct __align__(16) ItemDesc {
     float *ux, *uz;                          // adjoint displacement integrals
     float *glam, *gmu, *grho;                // [nfz][nfx]
     const float* fwd;                        // gradient source (see fwd_kind)
+    const int* evmap;                        // [ez1 - ez0 + 1][pitch] what happens in a cell (EvMap)
+    long long pad1;
 };
 
 struct Tile {
     int item, x0, z0, z1;
 };
+
+// Entry of a descriptor's event map: the kind in the two top bits, below it the
+// signal's row (one injection), the trace's row (one recording) or, for a cell
+// with several events, the index of its first one in ev.
+enum EvMap : unsigned { EV_NONE = 0u, EV_INJECT = 1u << 30, EV_RECORD = 2u << 30, EV_LIST = 3u << 30 };
 
 // CPML coefficient bundle of one strip index.
 struct Cpml {

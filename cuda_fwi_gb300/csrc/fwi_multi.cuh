@@ -40,6 +40,8 @@ struct MultiItem {
     int nfz, nfx, wz1;
     int nsrc, nrec;
     size_t evc_f, evc_a;  // offsets of the [nxt+1] column tables
+    int ez0[2], ez1[2];   // rows with events (forward, adjoint)
+    size_t off_map[2];    // offsets of the event maps
     int group;
 };
 
@@ -59,6 +61,8 @@ struct MultiEngine {
     DBuf d_fwd, d_adj, d_ws, d_wr, d_ux, d_uz, d_grad, d_mat, d_cpml, d_srcsig, d_rec, d_resid, d_obs;
     DBuf d_rowmis, d_blow, d_snap, d_items_f, d_items_a, d_evcol, d_ev, d_evx, d_err, d_rows;
     DBuf d_mmaps, d_gids;   // TMA maps per model; member lists of the groups (events)
+    DBuf d_evmap;           // event maps of every model, forward then adjoint
+    bool ev_map = false;    // the velocity passes of the TMA tiles inject and record
     bool mmaps_built = false;
     // Copy-free checkpointing (every group on the TMA tiles): buffer k < slots
     // is checkpoint memory, buffer `slots` is d_fwd; per buffer and model the
@@ -273,6 +277,29 @@ struct MultiEngine {
             CUDA_TRY(cudaMemcpy(d_evx.p, evx.data(), evx.size() * 4, cudaMemcpyHostToDevice));
         }
         FWI_TRY(d_rowmis.ensure(std::max<size_t>(1, nrows) * 8));
+        // event maps: per model and direction, the rows that hold events
+        std::vector<int> maps;
+        for (int b = 0; b < n; b++)
+            for (int adj = 0; adj < 2; adj++) {
+                MultiItem& I = items[b];
+                const int* c = cols_f.data() + (adj ? I.evc_a : I.evc_f);
+                int z0 = 0, z1 = -1;
+                for (int e = c[0]; e < c[I.nxt]; e++) {
+                    z0 = z1 < z0 ? ev_all[e].x : std::min(z0, ev_all[e].x);
+                    z1 = std::max(z1, ev_all[e].x);
+                }
+                I.ez0[adj] = z0;
+                I.ez1[adj] = z1;
+                I.off_map[adj] = maps.size();
+                maps.resize(maps.size() + (size_t)(z1 - z0 + 1) * I.pitch, 0);
+                fill_event_map(maps.data() + I.off_map[adj], z0, I.pitch, evx, ev_all, c[0], c[I.nxt]);
+            }
+        ev_map = maps.size() <= 8 * kEventMapMax;  // (made once per engine)
+        if (ev_map) {
+            FWI_TRY(d_evmap.ensure(std::max<size_t>(1, maps.size()) * 4));
+            if (!maps.empty())
+                CUDA_TRY(cudaMemcpy(d_evmap.p, maps.data(), maps.size() * 4, cudaMemcpyHostToDevice));
+        }
         // descriptors
         std::vector<ItemDesc> itf(n), ita(n);
         for (int b = 0; b < n; b++) {
@@ -424,6 +451,9 @@ struct MultiEngine {
         d.ev_col = d_evcol.as<int>() + (adj ? I.evc_a : I.evc_f);
         d.ev = d_ev.as<int2>();
         d.ev_x = d_evx.as<int>();
+        d.ez0 = I.ez0[adj];
+        d.ez1 = ev_map ? I.ez1[adj] : I.ez0[adj] - 1;
+        d.evmap = d_evmap.as<int>() + I.off_map[adj];
         d.inj = adj ? d_resid.as<float>() + I.off_rec : d_srcsig.as<float>() + I.off_src;
         d.rec = d_rec.as<float>() + I.off_rec;
         d.store = nullptr;
@@ -524,9 +554,12 @@ struct MultiEngine {
             const int ns = g.cum_f[k];
             const dim3 gs((unsigned)std::max(1, std::min(ns, num_sms)));
             g.tm.stress(gs, stream, mx, my, itm, g.tiles_f.as<Tile>(), ns, it, 0u, 0, msrc, err);
-            g.tm.velocity(gs, stream, mx, my, itm, g.tiles_f.as<Tile>(), ns, it, 0u, 0, msrc, err);
-            events_list_kernel<<<k, 256, 0, stream>>>(itm, d_gids.as<int>() + g.gid_off, it, FL_INJECT);
-            launches_now += 3;
+            g.tm.velocity(gs, stream, mx, my, itm, g.tiles_f.as<Tile>(), ns, it, FL_INJECT, 0, msrc, err);
+            launches_now += 2;
+            if (!ev_map) {
+                events_list_kernel<<<k, 256, 0, stream>>>(itm, d_gids.as<int>() + g.gid_off, it, FL_INJECT);
+                launches_now++;
+            }
         }
     }
     // The plan from action k on without state copies (the single-model
@@ -611,11 +644,11 @@ struct MultiEngine {
             }
             const int nv = g.cum_f[k];
             if (g.tune.fmap == 3) {
-                // source injection / recording of the active members in a small kernel after the pass
+                // without an event map, injection / recording of the active members in a kernel after the pass
                 const unsigned ev = vflags & (FL_INJECT | FL_RECORD);
                 g.tm.velocity(dim3((unsigned)std::max(1, std::min(nv, num_sms))), stream, mm, mm, itm,
-                              g.tiles_f.as<Tile>(), nv, it, vflags & ~ev, adj ? 1 : 0, 0, err);
-                if (ev) {
+                              g.tiles_f.as<Tile>(), nv, it, vflags, adj ? 1 : 0, 0, err);
+                if (ev && !ev_map) {
                     events_list_kernel<<<k, 256, 0, stream>>>(itm, d_gids.as<int>() + g.gid_off, it, ev);
                     launches_now++;
                 }
@@ -758,10 +791,11 @@ struct MultiEngine {
                 const dim3 gs((unsigned)std::max(1, std::min(ns, num_sms)));
                 g.tm.stress(gs, stream, mm, mm, d_items_f.as<ItemDesc>(), g.tiles_f.as<Tile>(), ns, 0, 0u, 0, 0,
                             d_err.as<int>());
-                g.tm.velocity(gs, stream, mm, mm, d_items_f.as<ItemDesc>(), g.tiles_f.as<Tile>(), ns, 0, 0u, 0, 0,
-                              d_err.as<int>());
-                events_list_kernel<<<k, 256, 0, stream>>>(d_items_f.as<ItemDesc>(), d_gids.as<int>() + g.gid_off, 0,
-                                                          FL_INJECT);
+                g.tm.velocity(gs, stream, mm, mm, d_items_f.as<ItemDesc>(), g.tiles_f.as<Tile>(), ns, 0, FL_INJECT, 0,
+                              0, d_err.as<int>());
+                if (!ev_map)
+                    events_list_kernel<<<k, 256, 0, stream>>>(d_items_f.as<ItemDesc>(), d_gids.as<int>() + g.gid_off,
+                                                              0, FL_INJECT);
             } else if (what == 1 && g.tune.amap == 3) {
                 const int ns = g.cum_a[k];
                 g.tm.adjoint(dim3((unsigned)std::max(1, std::min(ns, num_sms))), stream, mm, mm,

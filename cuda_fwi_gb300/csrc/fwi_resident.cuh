@@ -11,11 +11,11 @@
 //
 // What bounds the launch-per-pass schedule on small grids is not bandwidth: a
 // pass of the 244 x 244 grid takes ~4.5 us (launch, descriptor and tensor-map
-// fetches, one tile's copy latency), three launches per step.  Here a pass
+// fetches, one tile's copy latency), two launches per step.  Here a pass
 // costs its shared-memory stencil and one halo exchange.  Measured, us per
-// forward step, launches -> resident: 200x200 order 4 12.1 -> 3.1, 600x380
-// order 8 16.3 -> 5.7, 800x400 order 8 20.0 -> 8.7; adjoint steps over a stored
-// wavefield 200x200 17.6 -> 4.6.  What bounds it now: about 1.1 us of exchange
+// forward step, launches -> resident: 200x200 order 4 9.5 -> 3.1, 600x380
+// order 8 13.7 -> 5.7, 800x400 order 8 17.6 -> 8.7; adjoint steps over a stored
+// wavefield 200x200 15.8 -> 4.6.  What bounds it now: about 1.1 us of exchange
 // latency per pass, and above two rows per thread the shared-memory loads of the
 // stencil (31 per pair of cells) at 16 warps per SM.
 //

@@ -588,6 +588,61 @@ __device__ __forceinline__ void velocity_issue2(const VelMaps& ms, const VelMaps
     if (we) tma_load_3d(c + 4 * G::CEN, &mv.We, x0, z0, b, bar);
 }
 
+// The events of a cell after its velocity update (m: its entry of the event
+// map): injections in event order, then recordings of the result.
+__device__ __forceinline__ float cell_events(const ItemDesc& D, unsigned m, float v, int it, unsigned flags) {
+    const size_t nt = (size_t)D.nt;
+    const unsigned k = m & (EV_INJECT - 1u);
+    switch (m & EV_LIST) {
+        case EV_INJECT:
+            if (flags & FL_INJECT) v += __ldg(D.inj + k * nt + it);
+            break;
+        case EV_RECORD:
+            if (flags & FL_RECORD) D.rec[k * nt + it] = v;
+            break;
+        case EV_LIST: {
+            const int end = D.ev_col[D.nxt], x = D.ev_x[k];
+            const int2 first = D.ev[k];
+            for (int e = (int)k; e < end && D.ev_x[e] == x && D.ev[e].x == first.x; e++) {
+                const int code = D.ev[e].y;
+                if (code >= 0) {
+                    if (flags & FL_INJECT) v += __ldg(D.inj + code * nt + it);
+                } else if (flags & FL_RECORD) {
+                    D.rec[(size_t)(~code) * nt + it] = v;
+                }
+            }
+            break;
+        }
+    }
+    return v;
+}
+// The events of the cells that logical thread lt has just updated.  Not
+// inlined: in the velocity pass's loops this code cost the whole pass 2-3 %
+// (registers), and only the warps of the rows with events come here.
+static __device__ __noinline__ void pair_events(const ItemDesc* d, int x0, int z0, int lt, int it, unsigned flags) {
+    const ItemDesc& D = *d;
+    const int ix = x0 + (lt & (kTmaTX / 2 - 1)) * 2, P = D.pitch;
+    const int r = z0 + (lt / (kTmaTX / 2)) * kPairRows;
+    if (ix >= D.nxt) return;
+#pragma unroll
+    for (int rr = 0; rr < kPairRows; rr++) {
+        const int iz = r + rr;
+        if (iz < D.ez0 || iz > D.ez1) continue;
+        const long long i = (long long)(iz - D.ez0) * P + ix;
+        if (!inb(i + 1, (long long)(D.ez1 - D.ez0 + 1) * P, 25)) continue;
+        const int2 m = __ldg(reinterpret_cast<const int2*>(D.evmap + i));
+        float* vz = D.vz + (size_t)iz * P + ix;
+        if (m.x) {
+            const float v = vz[0], w = cell_events(D, (unsigned)m.x, v, it, flags);
+            if (w != v) vz[0] = w;
+        }
+        if (m.y) {
+            const float v = vz[1], w = cell_events(D, (unsigned)m.y, v, it, flags);
+            if (w != v) vz[1] = w;
+        }
+    }
+}
+
 template <int FP, bool INTERIOR>
 __device__ __forceinline__ void velocity_rows(const ItemDesc& D, const float* st, int x0, int z0, unsigned flags,
                                               const float2 (&hx)[FP], const float2 (&hz)[FP], long long msrc,
@@ -712,14 +767,18 @@ __device__ __forceinline__ void velocity_rows(const ItemDesc& D, const float* st
     }
 }
 
-// Source injection and receiver recording are not done here: the engine runs
-// them in a separate small kernel after this pass (events_kernel).
+// Source injection and receiver recording follow here where the descriptors
+// carry an event map and the flags ask for it, by the threads that own the
+// cells.  Without a map (events spread over too many rows) the engine runs
+// events_kernel after this pass: a launch of its own, 2-3 us per time step.
 template <int FP>
 __device__ __forceinline__ void velocity_compute(const ItemDesc& D, const TmaGrid& g, const float* st, int x0,
-                                                 int z0, unsigned flags, const float2 (&hx)[FP],
+                                                 int z0, int it, unsigned flags, const float2 (&hx)[FP],
                                                  const float2 (&hz)[FP], int lt) {
     if (interior_warp(g, x0, z0, flags, lt)) velocity_rows<FP, true>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
     else velocity_rows<FP, false>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
+    const int wz0 = z0 + (lt >> 6) * 2;
+    if ((flags & (FL_INJECT | FL_RECORD)) && wz0 <= D.ez1 && wz0 + 1 >= D.ez0) pair_events(&D, x0, z0, lt, it, flags);
 }
 
 // Stencil weights of a launch (every slot of a launch has the same grid),
@@ -912,8 +971,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             velocity_issue<FP>(maps, items + b, b, x0, z0, st, bar, we);
         },
         [&](int4 c, int4, const float* st, int k) {
-            velocity_compute<FP>(*reinterpret_cast<const ItemDesc*>(st + G::V_DESC), g, st, c.y, c.z, flags, hx, hz,
-                                 rotated_thread(k));
+            velocity_compute<FP>(*reinterpret_cast<const ItemDesc*>(st + G::V_DESC), g, st, c.y, c.z, it, flags, hx,
+                                 hz, rotated_thread(k));
         },
         g.wait_ns);
 }
@@ -1360,7 +1419,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             staged_weights<FP>(D, hx, hz);
             TmaGrid gg = model_ranges(D);
             gg.msrc = msrc;
-            velocity_compute<FP>(D, gg, st, c.y, c.z, flags, hx, hz, rotated_thread(k));
+            velocity_compute<FP>(D, gg, st, c.y, c.z, it, flags, hx, hz, rotated_thread(k));
         });
 }
 
