@@ -392,6 +392,24 @@ static KernelSet kernels_for(int fp, int map) {
     return map ? kernels_for_map<1>(fp) : kernels_for_map<0>(fp);
 }
 
+// Launch of a TMA-staged pass that may start while the kernel before it in the
+// stream drains (programmatic stream serialization; the pass itself waits for
+// that kernel's results, pass_begin in fwi_tma.cuh).
+template <class... P, class... A>
+static void launch_pass(void (*kernel)(P...), dim3 g, int threads, size_t smem, cudaStream_t s, const A&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = g;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // TMA-staged forward stress and velocity passes (fwi_tma.cuh).
 using TmaStressFn = void (*)(dim3, cudaStream_t, const StressMaps&, const ItemDesc*, TmaGrid, int, unsigned, int*);
 using TmaVelFn = void (*)(dim3, cudaStream_t, const VelMaps&, const ItemDesc*, TmaGrid, int, unsigned, int*);
@@ -405,17 +423,17 @@ struct TmaSet {
 template <int FP>
 static void t_stress(dim3 g, cudaStream_t s, const StressMaps& m, const ItemDesc* it, TmaGrid tg, int step,
                      unsigned flags, int* err) {
-    stress_tma_kernel<FP><<<g, kFwdThreads, stress_tma_smem<FP>(), s>>>(m, it, tg, step, flags, err);
+    launch_pass(stress_tma_kernel<FP>, g, kFwdThreads, stress_tma_smem<FP>(), s, m, it, tg, step, flags, err);
 }
 template <int FP>
 static void t_velocity(dim3 g, cudaStream_t s, const VelMaps& m, const ItemDesc* it, TmaGrid tg, int step,
                        unsigned flags, int* err) {
-    velocity_tma_kernel<FP><<<g, kFwdThreads, velocity_tma_smem<FP>(), s>>>(m, it, tg, step, flags, err);
+    launch_pass(velocity_tma_kernel<FP>, g, kFwdThreads, velocity_tma_smem<FP>(), s, m, it, tg, step, flags, err);
 }
 template <int FP>
 static void t_adjoint(dim3 g, cudaStream_t s, const AdjMaps& m, const ItemDesc* it, TmaGrid tg, int step,
                       unsigned flags, int* err) {
-    adjoint_tma_kernel<FP><<<g, kAdjThreads, adjoint_tma_smem<FP>(), s>>>(m, it, tg, step, flags, err);
+    launch_pass(adjoint_tma_kernel<FP>, g, kAdjThreads, adjoint_tma_smem<FP>(), s, m, it, tg, step, flags, err);
 }
 template <int FP>
 static cudaError_t t_prepare() {
@@ -503,19 +521,19 @@ struct TmaMultiSet {
 template <int FP>
 static void tm_stress(dim3 g, cudaStream_t s, const MultiMaps* mx, const MultiMaps* my, const ItemDesc* it,
                       const Tile* t, int nt, int step, unsigned flags, int, long long msrc, int* err) {
-    stress_tma_multi_kernel<FP><<<g, kFwdThreads, stress_tma_smem<FP>(), s>>>(mx, my, it, t, nt, step, flags, msrc,
-                                                                                 err);
+    launch_pass(stress_tma_multi_kernel<FP>, g, kFwdThreads, stress_tma_smem<FP>(), s, mx, my, it, t, nt, step, flags,
+                msrc, err);
 }
 template <int FP>
 static void tm_velocity(dim3 g, cudaStream_t s, const MultiMaps* mx, const MultiMaps* my, const ItemDesc* it,
                         const Tile* t, int nt, int step, unsigned flags, int adj, long long msrc, int* err) {
-    velocity_tma_multi_kernel<FP><<<g, kFwdThreads, velocity_tma_smem<FP>(), s>>>(mx, my, it, t, nt, step, flags,
-                                                                                     adj, msrc, err);
+    launch_pass(velocity_tma_multi_kernel<FP>, g, kFwdThreads, velocity_tma_smem<FP>(), s, mx, my, it, t, nt, step,
+                flags, adj, msrc, err);
 }
 template <int FP>
 static void tm_adjoint(dim3 g, cudaStream_t s, const MultiMaps* mx, const MultiMaps*, const ItemDesc* it,
                        const Tile* t, int nt, int step, unsigned flags, int, long long, int* err) {
-    adjoint_tma_multi_kernel<FP><<<g, kAdjThreads, adjoint_tma_smem<FP>(), s>>>(mx, it, t, nt, step, flags, err);
+    launch_pass(adjoint_tma_multi_kernel<FP>, g, kAdjThreads, adjoint_tma_smem<FP>(), s, mx, it, t, nt, step, flags, err);
 }
 template <int FP>
 static cudaError_t tm_prepare() {

@@ -822,6 +822,18 @@ __host__ __device__ constexpr size_t tma_tail_bytes() {
     return STAGES * (2 * sizeof(int4) + sizeof(uint64_t) + 2 * sizeof(unsigned)) + 16;
 }
 
+// Overlap with the neighbouring launches of the stream: the next pass's CTAs may
+// take this one's SMs as they fall free, and this pass waits here for the one
+// before it (whose results, and error word, it reads from now on).  What is
+// hidden is the launch and the barriers' set-up, ~2 us of a small pass: one shot
+// of 1068x568, order 8, stress 11.9 -> 9.5 us, velocity 10.3 -> 8.4 launch by
+// launch; inside graphs, where launches are closer, three shots of 547x269 order
+// 6 13.87 -> 13.41 ms a gradient, six of 463x343 order 12 5.09 -> 4.87 ms.
+__device__ __forceinline__ void pass_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned atom_add_acq_rel_cta(unsigned* p, unsigned v) {
     unsigned old;
     asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;"
@@ -846,6 +858,16 @@ __device__ __forceinline__ void tma_pipeline(int ntiles, int* err, Coords coords
     volatile int* abort = reinterpret_cast<volatile int*>(issued + S);
     const int tid = threadIdx.x, lane = tid & 31;
     const unsigned nwarps = blockDim.x >> 5;
+    if (tid == 0) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(&bar[s], 1);
+            released[s] = 0u;
+            issued[s] = 0u;
+        }
+        *abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pass_begin();
     // an earlier launch gave up (error word set): return at once, so a failing
     // pipeline costs one bounded wait and not one per launch; the decision is
     // CTA-uniform (every thread reaches the barrier)
@@ -872,13 +894,6 @@ __device__ __forceinline__ void tma_pipeline(int ntiles, int* err, Coords coords
         issue(b, x0, z0, tma_smem + s * STAGE_FLOATS, &bar[s]);
     };
     if (tid == 0) {
-        for (int s = 0; s < S; s++) {
-            mbar_init(&bar[s], 1);
-            released[s] = 0u;
-            issued[s] = 0u;
-        }
-        *abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (stall && blockIdx.x == 0) mbar_expect_tx_only(&bar[0], 16u);
         for (int s = 0; s < S; s++) {
             const int t = first + s * step;
