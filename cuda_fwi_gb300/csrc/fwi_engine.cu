@@ -1663,9 +1663,9 @@ struct Engine {
         fg.stall = stall_pending ? 1 : 0;
         stall_pending = false;
         const ItemDesc* items = d_items_b.as<ItemDesc>() + (size_t)y * B;
-        fset.step(dim3(grid_fused), stream, fmaps_b[x], items, fg, it, flags, d_err.as<int>());
+        fset.step(dim3(grid_fused), stream, fmaps_b[x], items, fg, it, flags | ev, d_err.as<int>());
         launches_now++;
-        if (ev) {
+        if (ev && !ev_map) {
             events_kernel<<<B, 256, 0, stream>>>(items, it, ev);
             launches_now++;
         }

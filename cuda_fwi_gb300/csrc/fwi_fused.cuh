@@ -554,6 +554,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             fused_velocity<FP, true>(D, st, ns, x0, qb, flags, hx, hz, g.msrc);
         else
             fused_velocity<FP, false>(D, st, ns, x0, qb, flags, hx, hz, g.msrc);
+        // sources and receivers, as after the two-pass step's velocities
+        const int cv = (tid & 63) * 2 - G::HX, r = qb + (w >> 1) * 2;
+        if ((flags & (FL_INJECT | FL_RECORD)) && r <= D.ez1 && r + 1 >= D.ez0 && cv >= 0 && cv < G::W)
+            pair_events(&D, x0 + cv, r, it, flags);
     }
 }
 

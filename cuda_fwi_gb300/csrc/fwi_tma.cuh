@@ -616,13 +616,12 @@ __device__ __forceinline__ float cell_events(const ItemDesc& D, unsigned m, floa
     }
     return v;
 }
-// The events of the cells that logical thread lt has just updated.  Not
-// inlined: in the velocity pass's loops this code cost the whole pass 2-3 %
+// The events of a column pair in rows [r, r + kPairRows) that this thread has
+// just updated.  Not inlined: in the velocity pass's loops this code cost the whole pass 2-3 %
 // (registers), and only the warps of the rows with events come here.
-static __device__ __noinline__ void pair_events(const ItemDesc* d, int x0, int z0, int lt, int it, unsigned flags) {
+static __device__ __noinline__ void pair_events(const ItemDesc* d, int ix, int r, int it, unsigned flags) {
     const ItemDesc& D = *d;
-    const int ix = x0 + (lt & (kTmaTX / 2 - 1)) * 2, P = D.pitch;
-    const int r = z0 + (lt / (kTmaTX / 2)) * kPairRows;
+    const int P = D.pitch;
     if (ix >= D.nxt) return;
 #pragma unroll
     for (int rr = 0; rr < kPairRows; rr++) {
@@ -778,7 +777,8 @@ __device__ __forceinline__ void velocity_compute(const ItemDesc& D, const TmaGri
     if (interior_warp(g, x0, z0, flags, lt)) velocity_rows<FP, true>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
     else velocity_rows<FP, false>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
     const int wz0 = z0 + (lt >> 6) * 2;
-    if ((flags & (FL_INJECT | FL_RECORD)) && wz0 <= D.ez1 && wz0 + 1 >= D.ez0) pair_events(&D, x0, z0, lt, it, flags);
+    if ((flags & (FL_INJECT | FL_RECORD)) && wz0 <= D.ez1 && wz0 + 1 >= D.ez0)
+        pair_events(&D, x0 + (lt & (kTmaTX / 2 - 1)) * 2, wz0, it, flags);
 }
 
 // Stencil weights of a launch (every slot of a launch has the same grid),
