@@ -598,46 +598,22 @@ static int make_map(CUtensorMap* m, const float* base, int nx, int nz, int nb, s
     return FWI_OK;
 }
 
-// Exact discrete adjoint (fwi_exact.cuh): four cell-parallel kernels per
+// Exact discrete adjoint (fwi_exact.cuh): two cell-parallel kernels per
 // reverse step plus the final chain rule onto lam, mu, rho.
 constexpr int kExactThreads = 256;
 constexpr int kDefaultMap = 3;  // thread mapping of a new engine (TMA-staged tiles)
-using ExactStepFn = void (*)(dim3, cudaStream_t, const ItemDesc*, const ExactDesc*, int, int, long long);
 struct ExactSet {
-    ExactStepFn vel_local, vel_stencil, str_local, str_stencil;
+    void (*velocity)(ExactArgs);
+    void (*stress)(ExactArgs);
 };
-template <int FP>
-static void x_vel_local(dim3 g, cudaStream_t s, const ItemDesc* it, const ExactDesc* ex, int nb, int step,
-                        long long cells) {
-    vel_adj_local<FP><<<g, kExactThreads, 0, s>>>(it, ex, nb, step, cells);
-}
-template <int FP>
-static void x_vel_stencil(dim3 g, cudaStream_t s, const ItemDesc* it, const ExactDesc* ex, int nb, int,
-                          long long cells) {
-    vel_adj_stencil<FP><<<g, kExactThreads, 0, s>>>(it, ex, nb, cells);
-}
-template <int FP>
-static void x_str_local(dim3 g, cudaStream_t s, const ItemDesc* it, const ExactDesc* ex, int nb, int,
-                        long long cells) {
-    str_adj_local<FP><<<g, kExactThreads, 0, s>>>(it, ex, nb, cells);
-}
-template <int FP>
-static void x_str_stencil(dim3 g, cudaStream_t s, const ItemDesc* it, const ExactDesc* ex, int nb, int,
-                          long long cells) {
-    str_adj_stencil<FP><<<g, kExactThreads, 0, s>>>(it, ex, nb, cells);
-}
-template <int FP>
-static ExactSet exact_set() {
-    return {x_vel_local<FP>, x_vel_stencil<FP>, x_str_local<FP>, x_str_stencil<FP>};
-}
 static ExactSet exact_for(int fp) {
     switch (fp) {
-        case 1: return exact_set<1>();
-        case 2: return exact_set<2>();
-        case 3: return exact_set<3>();
-        case 4: return exact_set<4>();
-        case 5: return exact_set<5>();
-        default: return exact_set<6>();
+        case 1: return {exact_velocity<1>, exact_stress<1>};
+        case 2: return {exact_velocity<2>, exact_stress<2>};
+        case 3: return {exact_velocity<3>, exact_stress<3>};
+        case 4: return {exact_velocity<4>, exact_stress<4>};
+        case 5: return {exact_velocity<5>, exact_stress<5>};
+        default: return {exact_velocity<6>, exact_stress<6>};
     }
 }
 
@@ -768,7 +744,7 @@ struct Engine {
     int ez0_f = 0, ez1_f = -1, ez0_a = 0, ez1_a = -1;
     bool ev_map = false;        // the velocity passes inject and record
     // exact discrete adjoint: forward state n+1, derivative adjoints + sensitivities, descriptors
-    DBuf d_nxt, d_exact, d_exd, d_items_n;
+    DBuf d_nxt, d_exact, d_exd, d_items_n, d_exh;
     ExactSet xs{};
     // TMA mapping: kernels, tensor maps per state buffer (0 fwd, 1 adj, 2 state n+1,
     // 3 fwd with the random-boundary materials), tile grid
@@ -1225,9 +1201,13 @@ struct Engine {
             if (d_snap.bytes != before) CUDA_TRY(cudaMemsetAsync(d_snap.p, 0, d_snap.bytes, stream));
         }
         if (exact()) {
+            // (border cells, which no pass writes, read as zero in every state buffer)
+            const size_t before = d_nxt.bytes;
             FWI_TRY(grow(d_nxt, (size_t)cap * state * 4));
+            if (d_nxt.bytes != before) CUDA_TRY(cudaMemsetAsync(d_nxt.p, 0, d_nxt.bytes, stream));
             FWI_TRY(grow(d_exact, (size_t)cap * 9 * field * 4));
             FWI_TRY(grow(d_exd, (size_t)cap * sizeof(ExactDesc)));
+            if (3 * nf < field) FWI_TRY(grow(d_exh, (size_t)cap * field * 4));
             FWI_TRY(grow(d_items_n, (size_t)cap * sizeof(ItemDesc)));
         }
         rows_cap = std::max(rows_cap, std::max<size_t>(1, nrows));
@@ -1347,16 +1327,22 @@ struct Engine {
             if (exact()) {
                 fill_item(itn[b], b, false, d_nxt.as<float>());
                 ExactDesc& x = exd[b];
-                x.tmp = d_exact.as<float>() + (size_t)b * 9 * field;
-                x.acc = x.tmp + 4 * field;
-                x.next = d_nxt.as<float>() + (size_t)b * state;
+                float* const tmp = d_exact.as<float>() + (size_t)b * 9 * field;
+                for (int k = 0; k < 4; k++) x.g[k] = tmp + k * field;
+                x.acc = tmp + 4 * field;
+                // the second set of derivative adjoints lives in buffers that this
+                // gradient does not use otherwise (Wr reads as zero afterwards)
+                x.h[0] = d_ux.as<float>() + (size_t)b * field;
+                x.h[1] = d_uz.as<float>() + (size_t)b * field;
+                x.h[2] = d_wr.as<float>() + (size_t)b * field;
+                x.h[3] = 3 * nf >= field ? d_grad.as<float>() + (size_t)b * 3 * nf : d_exh.as<float>() + (size_t)b * field;
                 x.src_col = itf[b].ev_col;
                 x.src_ev = itf[b].ev;
                 x.src_sig = d_srcsig.as<float>();
                 x.field = (long long)field;
             }
         }
-        if (copy_free() || fused()) {
+        if (buffered()) {
             const int nbuf = nbufs();
             std::vector<ItemDesc> itb((size_t)nbuf * B);
             for (int k = 0; k < nbuf; k++)
@@ -1405,8 +1391,8 @@ struct Engine {
     // round trips to L2 and about two saves and restores of the state.
     ResPlan resident_plan(int mode) const {
         ResPlan best;
-        if (bx_req != 0 || tz_req != 0 || kmap != 3 || fuse || exact() || random_mode() || snap_interval > 0 ||
-            !rset.launch)
+        if (bx_req != 0 || tz_req != 0 || kmap != 3 || fuse || (exact() && mode != RES_FORWARD) || random_mode() ||
+            snap_interval > 0 || !rset.launch)
             return best;
         static constexpr double kRowUs[kMaxHalf] = {1.2, 1.2, 1.7, 1.8, 3.3, 3.8};
         const int pairs = res_pairs(nxt, fpad), nz = nzt - 2 * fpad, most = kResTX / 2;
@@ -1748,7 +1734,7 @@ struct Engine {
             FWI_TRY(make_map(&A.fszx, f + F_SZX * field, nxt, nzt, Bcap, rb, sb, kTmaTX, kAdjTZ));
             FWI_TRY(make_map(&A.fszz, f + F_SZZ * field, nxt, nzt, Bcap, rb, sb, kTmaTX, kAdjTZ));
         }
-        if (copy_free() || fused()) {
+        if (buffered()) {
             const int nbuf = nbufs();
             smaps_b.assign(nbuf, smaps[0]);
             vmaps_b.assign(nbuf, vmaps[0]);
@@ -2019,31 +2005,120 @@ struct Engine {
             step(true, it, sf, FL_INJECT | FL_WE);
         }
     }
-    // One reverse step of the exact discrete adjoint at time step n: the
-    // working forward state (d_fwd) holds state n; state n+1 is made from it
-    // in d_nxt by one more forward step, then the four transposed passes run.
-    int exact_step(int n) {
+    // Kernels of the exact discrete adjoint for reverse step n over the forward
+    // states n (fw) and n+1 (nx) of the batch.
+    void exact_launch(bool velocity, const float* fw, const float* nx, int n, bool stencil, bool local) {
+        ExactArgs a{};
+        a.items = d_items_a.as<ItemDesc>();
+        a.ex = d_exd.as<ExactDesc>();
+        a.fw = fw;
+        a.nx = nx;
+        a.state = (long long)state;
+        a.it = n;
+        a.stencil = stencil;
+        a.local = local;
+        const dim3 g((unsigned)((nxt - 2 * fpad + kExactX - 1) / kExactX),
+                     (unsigned)((nzt - 2 * fpad + kExactZ - 1) / kExactZ), (unsigned)B);
+        (velocity ? xs.velocity : xs.stress)<<<g, dim3(kExactX, kExactZ), 0, stream>>>(a);
+        launches_now++;
+    }
+    // After the last reverse step: its velocity stencils, then the chain rule (the
+    // buffers that held H read as zero again, but for the gradient's own).
+    int exact_finish() {
+        exact_launch(true, nullptr, nullptr, 0, true, false);
+        CUDA_TRY(cudaMemsetAsync(d_wr.p, 0, (size_t)B * field * 4, stream));
+        const dim3 g((unsigned)((nf + kExactThreads - 1) / kExactThreads), (unsigned)B);
+        chain_rule<<<g, kExactThreads, 0, stream>>>(d_items_a.as<ItemDesc>(), d_exd.as<ExactDesc>(), B);
+        launches_now++;
+        return FWI_OK;
+    }
+    // One reverse step where the states are copied (mappings other than the TMA
+    // one): the working forward state (d_fwd) holds state n; state n+1 is made
+    // from it in d_nxt by one more forward step.
+    int exact_step(int n, bool first) {
         FWI_TRY(state_copy(d_nxt.as<float>(), d_fwd.as<float>()));
         const ItemDesc* itn = d_items_n.as<ItemDesc>();
         pass_stress_fwd(2, itn, n, 0u);
         pass_velocity(2, itn, n, FL_INJECT);
-        const long long cells = (long long)(nzt - 2 * fpad) * (nxt - 2 * fpad);
-        const dim3 g((unsigned)((cells + kExactThreads - 1) / kExactThreads), (unsigned)B);
-        const ItemDesc* ia = d_items_a.as<ItemDesc>();
-        const ExactDesc* ex = d_exd.as<ExactDesc>();
-        xs.vel_local(g, stream, ia, ex, B, n, cells);
-        xs.vel_stencil(g, stream, ia, ex, B, n, cells);
-        xs.str_local(g, stream, ia, ex, B, n, cells);
-        xs.str_stencil(g, stream, ia, ex, B, n, cells);
-        launches_now += 6;
+        launches_now += 2;
+        exact_launch(true, d_fwd.as<float>(), d_nxt.as<float>(), n, !first, true);
+        exact_launch(false, d_fwd.as<float>(), d_nxt.as<float>(), n, false, false);
+        return FWI_OK;
+    }
+    // The binomial plan of the exact adjoint from action k on without state
+    // copies and without the extra forward step (TMA mapping).  A reverse step
+    // needs the states n and n+1, and n+1 is the state the previous reverse step
+    // started from (for the last one, the final state of the forward sweep), so
+    // its buffer is left alone until then.  Buffers: the checkpoint memory,
+    // d_fwd and d_nxt; own[] are those that hold a live checkpoint, `cur` the
+    // working state, `prev` state n+1.  A step goes in place when nobody else
+    // needs the buffer, otherwise into a free one (there is one: at most the
+    // slots, the working state and state n+1 are in use, and a state in a slot
+    // is not counted twice).
+    int run_plan_exact(size_t k, int last_slot, int last_state) {
+        const int nbuf = nbufs();
+        std::vector<int> own(slots, -1);
+        for (size_t i = 0; i < k; i++)
+            if (plan[i].kind == Action::SAVE) own[plan[i].a] = plan[i].a;
+        int prev = slots;  // d_fwd: the forward sweep's final state
+        int cur = -1;
+        auto owned = [&](int b) { return std::find(own.begin(), own.end(), b) != own.end(); };
+        auto free_buffer = [&]() {
+            for (int b = nbuf - 1; b >= 0; b--)
+                if (b != prev && b != cur && !owned(b)) return b;
+            return -1;
+        };
+        auto zero = [&]() -> int {
+            cur = -1;
+            const int b = free_buffer();
+            if (b < 0) return fail(FWI_ERR_STATE, "no free state buffer");
+            CUDA_TRY(cudaMemsetAsync(buf(b), 0, (size_t)B * state * 4, stream));
+            cur = b;
+            return FWI_OK;
+        };
+        auto advance = [&](int t0, int t1) -> int {
+            for (int it = t0; it < t1; it++) {
+                int dst = cur;
+                if (cur == prev || owned(cur)) dst = free_buffer();
+                if (dst < 0) return fail(FWI_ERR_STATE, "no free state buffer");
+                step_bufs(cur, dst, it);
+                cur = dst;
+            }
+            return FWI_OK;
+        };
+        if (last_slot >= 0) cur = own[last_slot];
+        else FWI_TRY(zero());
+        FWI_TRY(advance(last_state, nt - 1));
+        bool first = true;
+        for (; k < plan.size(); k++) {
+            const Action& a = plan[k];
+            switch (a.kind) {
+                case Action::ADVANCE:
+                    FWI_TRY(advance(a.a, a.b));
+                    break;
+                case Action::SAVE:
+                    own[a.a] = cur;
+                    break;
+                case Action::RESTORE:
+                    if (a.a < 0) FWI_TRY(zero());
+                    else cur = own[a.a];
+                    break;
+                case Action::ADJOINT:
+                    exact_launch(true, buf(cur), buf(prev), a.a, !first, true);
+                    exact_launch(false, buf(cur), buf(prev), a.a, false, false);
+                    first = false;
+                    prev = cur;
+                    break;
+            }
+        }
         return FWI_OK;
     }
     // Forward steps the backward runs for the plan (in units of fwi_dt): from
     // the last checkpoint of the first sweep (placed by forward()) to the last
-    // unit, then every ADVANCE after that prefix, plus state n+1 of each exact
-    // reverse step.  The same count whether the plan runs directly or as a
+    // unit, then every ADVANCE after that prefix, plus (where the exact adjoint
+    // copies states) state n+1 of each reverse step.  The same count whether the plan runs directly or as a
     // replayed graph.
-    long long plan_recompute() const { return plan_recompute_steps(plan, nunits(), exact()); }
+    long long plan_recompute() const { return plan_recompute_steps(plan, nunits(), exact() && kmap != 3); }
     int state_copy(float* dst, const float* src) {
         CUDA_TRY(device_copy(dst, src, (size_t)B * state, num_sms, stream));
         launches_now++;
@@ -2053,10 +2128,14 @@ struct Engine {
     // The binomial plan runs without state copies on the TMA mapping (the
     // other mappings and the exact adjoint copy states in and out of slots).
     bool copy_free() const { return kmap == 3 && ckpt_mode() && !exact() && slots > 0; }
-    float* buf(int k) { return k < slots ? snap(k) : k == slots ? d_fwd.as<float>() : d_fwd2.as<float>(); }
+    float* buf(int k) {
+        return k < slots ? snap(k) : k == slots ? d_fwd.as<float>() : exact() ? d_nxt.as<float>() : d_fwd2.as<float>();
+    }
+    // State buffers with maps and descriptors of their own (step_bufs).
+    bool buffered() const { return copy_free() || fused() || (kmap == 3 && exact()); }
     // Buffers a step can read or write: the checkpoint slots, d_fwd and, for
-    // the fused step, d_fwd2.
-    int nbufs() const { return slots + (fused() ? 2 : 1); }
+    // the fused step, d_fwd2, for the exact adjoint d_nxt.
+    int nbufs() const { return slots + (fused() || exact() ? 2 : 1); }
     // One recompute step (stress, velocity, source injection) from the state
     // of step `it` in buffer x to the state of step it+1 in buffer y (x == y:
     // in place).  Out of place, the stress pass reads velocities and
@@ -2310,7 +2389,10 @@ struct Engine {
             CUDA_TRY(cudaMemsetAsync(d_ux.p, 0, (size_t)B * field * 4, stream));
             CUDA_TRY(cudaMemsetAsync(d_uz.p, 0, (size_t)B * field * 4, stream));
             CUDA_TRY(cudaMemsetAsync(d_grad.p, 0, (size_t)B * 3 * nf * 4, stream));
-            if (exact()) CUDA_TRY(cudaMemsetAsync(d_exact.p, 0, (size_t)B * 9 * field * 4, stream));
+            if (exact()) {
+                CUDA_TRY(cudaMemsetAsync(d_exact.p, 0, (size_t)B * 9 * field * 4, stream));
+                if (d_exh.p) CUDA_TRY(cudaMemsetAsync(d_exh.p, 0, d_exh.bytes, stream));
+            }
             if (random_mode()) {
                 // reverse-time reconstruction of the source wavefield, one step
                 // ahead of the adjoint step that correlates with it
@@ -2343,6 +2425,11 @@ struct Engine {
                 FWI_TRY(run_plan_copy_free(k, last_slot, last_state));
                 return FWI_OK;
             }
+            if (exact() && kmap == 3) {
+                FWI_TRY(run_plan_exact(k, last_slot, last_state));
+                return exact_finish();
+            }
+            bool first = true;
             // working buffer: state of the last prefix checkpoint, advanced to nft-1
             if (last_slot >= 0) FWI_TRY(state_copy(d_fwd.as<float>(), snap(last_slot)));
             else CUDA_TRY(cudaMemsetAsync(d_fwd.p, 0, (size_t)B * state * 4, stream));
@@ -2364,7 +2451,8 @@ struct Engine {
                         break;
                     case Action::ADJOINT: {
                         if (exact()) {
-                            FWI_TRY(exact_step(a.a));
+                            FWI_TRY(exact_step(a.a, first));
+                            first = false;
                             recompute += 1;  // state n+1 of the reverse step
                             break;
                         }
@@ -2374,11 +2462,7 @@ struct Engine {
                     }
                 }
             }
-            if (exact()) {
-                const dim3 g((unsigned)((nf + kExactThreads - 1) / kExactThreads), (unsigned)B);
-                chain_rule<<<g, kExactThreads, 0, stream>>>(d_items_a.as<ItemDesc>(), d_exd.as<ExactDesc>(), B);
-                launches_now++;
-            }
+            if (exact()) FWI_TRY(exact_finish());
             return FWI_OK;
         }));
         if (pre_on) {

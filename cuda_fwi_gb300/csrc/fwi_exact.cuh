@@ -13,15 +13,22 @@
 //             szx += MZ (b_x' + a_z')
 //   velocity: c_x = Dx+ sxx, d_x = Dx- szx, d_z = Dz- szx, e_z = Dz+ szz (+ CPML)
 //             vx += BX (c_x' + d_z');  vz += BZ (d_x' + e_z') [+ source]
-// Reverse step n, given the adjoints of level n+1 (one kernel each):
-//   1. vel_adj_local: vz^-[rec] += dt (d_n - obs_n); w1 = BX vx^-, w2 = BZ vz^-;
-//      CPML transposes give the derivative adjoints G (4 fields); the
-//      sensitivities R += vx^- dvx, T += vz^- (dvz - src) accumulate.
-//   2. vel_adj_stencil: s^- += (D)^T G.
-//   3. str_adj_local: stress derivative adjoints + CPML transposes -> H (4
-//      fields); P += (sxx^- + szz^-)(dsxx + dszz), A += sxx^- dsxx + szz^- dszz,
+// Reverse step n, given the adjoints of level n+1:
+//   1. vz^-[rec] += dt (d_n - obs_n); w1 = BX vx^-, w2 = BZ vz^-; CPML transposes
+//      give the derivative adjoints G (4 fields); the sensitivities R += vx^- dvx,
+//      T += vz^- (dvz - src) accumulate.
+//   2. s^- += (D)^T G.
+//   3. stress derivative adjoints + CPML transposes -> H (4 fields);
+//      P += (sxx^- + szz^-)(dsxx + dszz), A += sxx^- dsxx + szz^- dszz,
 //      Q += szx^- dszx.
-//   4. str_adj_stencil: v^- += (D)^T H.
+//   4. v^- += (D)^T H.
+// 2 and 3 read other cells' G but only their own stresses, so they are one kernel
+// (exact_stress), and so are 4 of step n and 1 of step n-1 (exact_velocity): two
+// launches per reverse step.  G and H are zero on the border cells (cleared
+// before the sweep, never written there), so the stencils need no range checks.
+// Measured, 868x468 cells, order 8, us per reverse step with everything it needs
+// of the forward states: 88 as four kernels after a copy of state n and one more
+// forward step, 51 now.
 // Free surface (row fpad): the forward assigns sxx = c a_x' with
 // c = M2 (2L + M2)/(L + M2) and zeroes szx, szz there, then mirrors szx, szz of
 // rows fpad+1..2fpad onto rows fpad-1..0 with a minus sign.  The transpose
@@ -43,22 +50,32 @@ namespace fwi {
 
 // Adjoint-only buffers of one shot, reached through ExactDesc.
 struct ExactDesc {
-    float* tmp;            // [4][field] G or H derivative adjoints
+    float* g[4];           // G derivative adjoints [field]
+    float* h[4];           // H
     float* acc;            // [5][field] P, A, Q, R, T
-    const float* next;     // forward state n+1: [5][field] (vx, vz, sxx, szx, szz)
     const int* src_col;    // forward source events by column (inject codes only)
     const int2* src_ev;
     const float* src_sig;  // [nsrc][nt]
     long long field;       // floats per field
 };
 
-__device__ __forceinline__ bool cell_of(const ItemDesc& D, long long idx, int FPv, int* iz, int* ix) {
-    const int nxi = D.nxt - 2 * FPv;
-    const int nzi = D.nzt - 2 * FPv;
-    if (idx >= (long long)nxi * nzi) return false;
-    *iz = FPv + (int)(idx / nxi);
-    *ix = FPv + (int)(idx % nxi);
-    return true;
+// One launch: the forward states n and n+1 of the batch (shot b at b * state).
+struct ExactArgs {
+    const ItemDesc* items;
+    const ExactDesc* ex;
+    const float *fw, *nx;
+    long long state;
+    int it;                // n
+    int stencil, local;    // exact_velocity: parts 4 of the step before, 1 of this one
+};
+constexpr int kExactX = 64, kExactZ = 4;  // cells of a block
+
+// Interior cell of this thread (false: none).
+template <int FP>
+__device__ __forceinline__ bool cell_of(const ItemDesc& D, int* iz, int* ix) {
+    *ix = FP + (int)(blockIdx.x * kExactX + threadIdx.x);
+    *iz = FP + (int)(blockIdx.y * kExactZ + threadIdx.y);
+    return *ix < D.nxt - FP && *iz < D.nzt - FP;
 }
 
 // x / z strip indices of the two passes (same rules as the forward kernels).
@@ -100,130 +117,113 @@ __device__ __forceinline__ float cpml_adj(float ubar, float* m, float a, float b
     return ubar * iK + a * tot;
 }
 
+// Part 4 of the step before (velocity adjoints from H) and part 1 of step n.
 template <int FP>
-__global__ void vel_adj_local(const ItemDesc* __restrict__ items, const ExactDesc* __restrict__ ex, int nb,
-                              int it, long long cells) {
-    const int b = blockIdx.y;
-    if (b >= nb) return;
-    const ItemDesc& D = items[b];
-    const ExactDesc& E = ex[b];
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kExactX* kExactZ) exact_velocity(const ExactArgs A) {
+    const int b = blockIdx.z;
+    const ItemDesc& D = A.items[b];
+    const ExactDesc& E = A.ex[b];
     int iz, ix;
-    if (idx >= cells || !cell_of(D, idx, FP, &iz, &ix)) return;
+    if (!cell_of<FP>(D, &iz, &ix)) return;
     const int P = D.pitch, tp = D.tp;
     const size_t c = (size_t)iz * P + ix;
-    float vzb = D.vz[c];
-    const float vxb = D.vx[c];
-    // receivers record vz^{n+1} after the source: their adjoint source comes first
-    const int e1 = D.ev_col[ix + 1];
-    bool touched = false;
-    for (int e = D.ev_col[ix]; e < e1; e++) {
-        const int2 ev = D.ev[e];
-        if (ev.x == iz && ev.y >= 0) {
-            vzb += D.dt * D.inj[(size_t)ev.y * D.nt + it];
-            touched = true;
+    float vxb = D.vx[c], vzb = D.vz[c];
+    if (A.stencil) {
+        float vx = 0.f, vz = 0.f;
+#pragma unroll
+        for (int k = 1; k <= FP; k++) {
+            const float hx = D.hx[k - 1], hz = D.hz[k - 1];
+            vx += hx * (E.h[0][c - k + 1] - E.h[0][c + k]);                                         // (Dx-)^T
+            vx += hz * (E.h[2][c - (size_t)k * P] - E.h[2][c + (size_t)(k - 1) * P]);               // (Dz+)^T
+            vz += hx * (E.h[1][c - k] - E.h[1][c + k - 1]);                                         // (Dx+)^T
+            vz += hz * (E.h[3][c - (size_t)(k - 1) * P] - E.h[3][c + (size_t)k * P]);               // (Dz-)^T
         }
+        vxb += vx;
+        vzb += vz;
+        D.vx[c] = vxb;
     }
-    if (touched) D.vz[c] = vzb;
-    // sensitivities to BX, BZ: adjoint times the forward increment (minus the source)
-    const float* nx = E.next;
-    const float* fw = D.fwd;  // forward state n
-    const long long F = E.field;
-    const float dvx = nx[F_VX * F + c] - fw[F_VX * F + c];
-    float dvz = nx[F_VZ * F + c] - fw[F_VZ * F + c];
-    const int s1 = E.src_col[ix + 1];
-    for (int e = E.src_col[ix]; e < s1; e++) {
-        const int2 ev = E.src_ev[e];
-        if (ev.x == iz && ev.y >= 0) dvz -= E.src_sig[(size_t)ev.y * D.nt + it];
+    if (A.local) {
+        // receivers record vz^{n+1} after the source: their adjoint source comes first
+        const int e1 = D.ev_col[ix + 1];
+        for (int e = D.ev_col[ix]; e < e1; e++) {
+            const int2 ev = D.ev[e];
+            if (ev.x == iz && ev.y >= 0) vzb += D.dt * D.inj[(size_t)ev.y * D.nt + A.it];
+        }
+        // sensitivities to BX, BZ: adjoint times the forward increment (minus the source)
+        const long long F = E.field;
+        const float* nx = A.nx + b * A.state;
+        const float* fw = A.fw + b * A.state;
+        const float dvx = nx[F_VX * F + c] - fw[F_VX * F + c];
+        float dvz = nx[F_VZ * F + c] - fw[F_VZ * F + c];
+        const int s1 = E.src_col[ix + 1];
+        for (int e = E.src_col[ix]; e < s1; e++) {
+            const int2 ev = E.src_ev[e];
+            if (ev.x == iz && ev.y >= 0) dvz -= E.src_sig[(size_t)ev.y * D.nt + A.it];
+        }
+        E.acc[3 * F + c] += vxb * dvx;
+        E.acc[4 * F + c] += vzb * dvz;
+        const float w1 = D.BX[c] * vxb, w2 = D.BZ[c] * vzb;
+        // c_x (full, psi5 = msxx_x), d_x (half, psi6 = mszx_x) from w1 / w2; d_z (half, psi8), e_z (full, psi7)
+        float gcx = w1, gdx = w2, gdz = w1, gez = w2;
+        const float* cp = D.cpml;
+        const int px = velocity_px(D, ix, FP);
+        if (px >= 0) {
+            const size_t m = (size_t)iz * tp + px;
+            gcx = cpml_adj(w1, D.msxx_x + m, cp[px], cp[tp + px], cp[2 * tp + px]);
+            gdx = cpml_adj(w2, D.mszx_x + m, cp[3 * tp + px], cp[4 * tp + px], cp[5 * tp + px]);
+        }
+        const int pz = velocity_pz(D, iz, FP);
+        if (pz >= 0) {
+            const size_t m = (size_t)pz * P + ix;
+            gez = cpml_adj(w2, D.mszz_z + m, cp[pz], cp[tp + pz], cp[2 * tp + pz]);
+            gdz = cpml_adj(w1, D.mszx_z + m, cp[3 * tp + pz], cp[4 * tp + pz], cp[5 * tp + pz]);
+        }
+        E.g[0][c] = gcx;
+        E.g[1][c] = gdx;
+        E.g[2][c] = gdz;
+        E.g[3][c] = gez;
     }
-    E.acc[3 * F + c] += vxb * dvx;
-    E.acc[4 * F + c] += vzb * dvz;
-    const float w1 = D.BX[c] * vxb, w2 = D.BZ[c] * vzb;
-    // c_x (full, psi5 = msxx_x), d_x (half, psi6 = mszx_x) from w1 / w2; d_z (half, psi8), e_z (full, psi7)
-    float gcx = w1, gdx = w2, gdz = w1, gez = w2;
-    const float* cp = D.cpml;
-    const int px = velocity_px(D, ix, FP);
-    if (px >= 0) {
-        const size_t m = (size_t)iz * tp + px;
-        gcx = cpml_adj(w1, D.msxx_x + m, cp[px], cp[tp + px], cp[2 * tp + px]);
-        gdx = cpml_adj(w2, D.mszx_x + m, cp[3 * tp + px], cp[4 * tp + px], cp[5 * tp + px]);
-    }
-    const int pz = velocity_pz(D, iz, FP);
-    if (pz >= 0) {
-        const size_t m = (size_t)pz * P + ix;
-        gez = cpml_adj(w2, D.mszz_z + m, cp[pz], cp[tp + pz], cp[2 * tp + pz]);
-        gdz = cpml_adj(w1, D.mszx_z + m, cp[3 * tp + pz], cp[4 * tp + pz], cp[5 * tp + pz]);
-    }
-    E.tmp[0 * F + c] = gcx;
-    E.tmp[1 * F + c] = gdx;
-    E.tmp[2 * F + c] = gdz;
-    E.tmp[3 * F + c] = gez;
+    D.vz[c] = vzb;
 }
 
+// Parts 2 and 3 of step n: stress adjoints from G, then H.
 template <int FP>
-__device__ __forceinline__ float tmp_at(const ItemDesc& D, const float* t, int iz, int ix) {
-    // derivative adjoints live on interior cells only
-    if (iz < FP || iz >= D.nzt - FP || ix < FP || ix >= D.nxt - FP) return 0.f;
-    return t[(size_t)iz * D.pitch + ix];
-}
-
-template <int FP>
-__global__ void vel_adj_stencil(const ItemDesc* __restrict__ items, const ExactDesc* __restrict__ ex,
-                                int nb, long long cells) {
-    const int b = blockIdx.y;
-    if (b >= nb) return;
-    const ItemDesc& D = items[b];
-    const ExactDesc& E = ex[b];
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kExactX* kExactZ) exact_stress(const ExactArgs A) {
+    const int b = blockIdx.z;
+    const ItemDesc& D = A.items[b];
+    const ExactDesc& E = A.ex[b];
     int iz, ix;
-    if (idx >= cells || !cell_of(D, idx, FP, &iz, &ix)) return;
+    if (!cell_of<FP>(D, &iz, &ix)) return;
+    const int P = D.pitch, tp = D.tp;
+    const size_t c = (size_t)iz * P + ix;
     const long long F = E.field;
-    const float *gcx = E.tmp, *gdx = E.tmp + F, *gdz = E.tmp + 2 * F, *gez = E.tmp + 3 * F;
     float sxx = 0.f, szx = 0.f, szz = 0.f;
 #pragma unroll
     for (int k = 1; k <= FP; k++) {
         const float hx = D.hx[k - 1], hz = D.hz[k - 1];
-        sxx += hx * (tmp_at<FP>(D, gcx, iz, ix - k) - tmp_at<FP>(D, gcx, iz, ix + k - 1));       // (Dx+)^T
-        szx += hx * (tmp_at<FP>(D, gdx, iz, ix - k + 1) - tmp_at<FP>(D, gdx, iz, ix + k));       // (Dx-)^T
-        szx += hz * (tmp_at<FP>(D, gdz, iz - k + 1, ix) - tmp_at<FP>(D, gdz, iz + k, ix));       // (Dz-)^T
-        szz += hz * (tmp_at<FP>(D, gez, iz - k, ix) - tmp_at<FP>(D, gez, iz + k - 1, ix));       // (Dz+)^T
+        sxx += hx * (E.g[0][c - k] - E.g[0][c + k - 1]);                                         // (Dx+)^T
+        szx += hx * (E.g[1][c - k + 1] - E.g[1][c + k]);                                         // (Dx-)^T
+        szx += hz * (E.g[2][c - (size_t)(k - 1) * P] - E.g[2][c + (size_t)k * P]);               // (Dz-)^T
+        szz += hz * (E.g[3][c - (size_t)k * P] - E.g[3][c + (size_t)(k - 1) * P]);               // (Dz+)^T
     }
     if (D.fsurf && iz > FP && iz <= 2 * FP) {
         // rows fpad-1..0 hold -szx, -szz of rows fpad+1..2fpad: their adjoints
         // (z-stencil taps of the interior rows only) fold back with a minus sign
         const int r = 2 * FP - iz;
+        auto at = [&](const float* g, int z) { return z < FP ? 0.f : g[(size_t)z * P + ix]; };
         float px = 0.f, pz = 0.f;
 #pragma unroll
         for (int k = 1; k <= FP; k++) {
             const float hz = D.hz[k - 1];
-            px += hz * (tmp_at<FP>(D, gdz, r - k + 1, ix) - tmp_at<FP>(D, gdz, r + k, ix));
-            pz += hz * (tmp_at<FP>(D, gez, r - k, ix) - tmp_at<FP>(D, gez, r + k - 1, ix));
+            px += hz * (at(E.g[2], r - k + 1) - at(E.g[2], r + k));
+            pz += hz * (at(E.g[3], r - k) - at(E.g[3], r + k - 1));
         }
         szx -= px;
         szz -= pz;
     }
-    const size_t c = (size_t)iz * D.pitch + ix;
-    D.sxx[c] += sxx;
-    D.szx[c] += szx;
-    D.szz[c] += szz;
-}
-
-template <int FP>
-__global__ void str_adj_local(const ItemDesc* __restrict__ items, const ExactDesc* __restrict__ ex, int nb,
-                              long long cells) {
-    const int b = blockIdx.y;
-    if (b >= nb) return;
-    const ItemDesc& D = items[b];
-    const ExactDesc& E = ex[b];
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int iz, ix;
-    if (idx >= cells || !cell_of(D, idx, FP, &iz, &ix)) return;
-    const int P = D.pitch, tp = D.tp;
-    const size_t c = (size_t)iz * P + ix;
-    const long long F = E.field;
-    const float sxxb = D.sxx[c], szxb = D.szx[c], szzb = D.szz[c];
-    const float* nx = E.next;
-    const float* fw = D.fwd;
+    const float sxxb = D.sxx[c] + sxx, szxb = D.szx[c] + szx, szzb = D.szz[c] + szz;
+    const float* nx = A.nx + b * A.state;
+    const float* fw = A.fw + b * A.state;
     const float L = D.L[c], M2 = D.M2[c], MZ = D.MZX[c];
     float ax, bz, bx, az;  // adjoints of a_x' (vx_x), b_z' (vz_z), b_x' (vz_x), a_z' (vx_z)
     if (D.fsurf && iz == FP) {
@@ -249,6 +249,9 @@ __global__ void str_adj_local(const ItemDesc* __restrict__ items, const ExactDes
         bz = L * sxxb + (L + M2) * szzb;
         bx = MZ * szxb;
         az = MZ * szxb;
+        D.sxx[c] = sxxb;
+        D.szx[c] = szxb;
+        D.szz[c] = szzb;
     }
     float hax = ax, hbx = bx, haz = az, hbz = bz;
     const float* cp = D.cpml;
@@ -264,36 +267,10 @@ __global__ void str_adj_local(const ItemDesc* __restrict__ items, const ExactDes
         hbz = cpml_adj(bz, D.mvz_z + m, cp[pz], cp[tp + pz], cp[2 * tp + pz]);
         haz = cpml_adj(az, D.mvx_z + m, cp[3 * tp + pz], cp[4 * tp + pz], cp[5 * tp + pz]);
     }
-    E.tmp[0 * F + c] = hax;
-    E.tmp[1 * F + c] = hbx;
-    E.tmp[2 * F + c] = haz;
-    E.tmp[3 * F + c] = hbz;
-}
-
-template <int FP>
-__global__ void str_adj_stencil(const ItemDesc* __restrict__ items, const ExactDesc* __restrict__ ex,
-                                int nb, long long cells) {
-    const int b = blockIdx.y;
-    if (b >= nb) return;
-    const ItemDesc& D = items[b];
-    const ExactDesc& E = ex[b];
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int iz, ix;
-    if (idx >= cells || !cell_of(D, idx, FP, &iz, &ix)) return;
-    const long long F = E.field;
-    const float *hax = E.tmp, *hbx = E.tmp + F, *haz = E.tmp + 2 * F, *hbz = E.tmp + 3 * F;
-    float vx = 0.f, vz = 0.f;
-#pragma unroll
-    for (int k = 1; k <= FP; k++) {
-        const float hx = D.hx[k - 1], hz = D.hz[k - 1];
-        vx += hx * (tmp_at<FP>(D, hax, iz, ix - k + 1) - tmp_at<FP>(D, hax, iz, ix + k));   // (Dx-)^T
-        vx += hz * (tmp_at<FP>(D, haz, iz - k, ix) - tmp_at<FP>(D, haz, iz + k - 1, ix));   // (Dz+)^T
-        vz += hx * (tmp_at<FP>(D, hbx, iz, ix - k) - tmp_at<FP>(D, hbx, iz, ix + k - 1));   // (Dx+)^T
-        vz += hz * (tmp_at<FP>(D, hbz, iz - k + 1, ix) - tmp_at<FP>(D, hbz, iz + k, ix));   // (Dz-)^T
-    }
-    const size_t c = (size_t)iz * D.pitch + ix;
-    D.vx[c] += vx;
-    D.vz[c] += vz;
+    E.h[0][c] = hax;
+    E.h[1][c] = hbx;
+    E.h[2][c] = haz;
+    E.h[3][c] = hbz;
 }
 
 // Sensitivities to the dt-scaled materials -> gradients of lam, mu, rho on the
