@@ -40,9 +40,8 @@ MODES = ("exact", "reference")
 def _to_grid(g, p):
     """[nfz][nfx] window gradient -> [nzt][nxt] grid (zeros outside the window)."""
     out = np.zeros((p.nzt, p.nxt))
-    zs = np.arange(p.z1, p.z2, p.fwi_dz)
-    xs = np.arange(p.x1, p.x2, p.fwi_dx)
-    out[np.ix_(zs, xs)] = g[: len(zs), : len(xs)]
+    window = out[p.z1:p.z2:p.fwi_dz, p.x1:p.x2:p.fwi_dx]
+    window[...] = g[: window.shape[0], : window.shape[1]]
     return out
 
 

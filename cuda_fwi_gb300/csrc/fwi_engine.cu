@@ -940,18 +940,20 @@ struct Engine {
         float* MZ = M2 + field;
         float* BXp = MZ + field;
         float* BZp = BXp + field;
-        for (int iz = 0; iz < nzt; iz++)
-            for (int ix = 0; ix < nxt; ix++) {
-                const size_t o = (size_t)iz * pitch + ix, c = (size_t)iz * nxt + ix;
-                L[o] = (float)(dt * lam[c]);
-                M2[o] = (float)(2.0 * dt * mu[c]);
-                if (iz < nzt - 1 && ix < nxt - 1) {
-                    const size_t a = (size_t)iz * (nxt - 1) + ix;
-                    MZ[o] = (float)(dt * mu_zx[a]);
-                    BXp[o] = (float)(dt * rho_xp[a]);
-                    BZp[o] = (float)(dt * rho_zp[a]);
+        parallel_for(nzt, std::max<size_t>(1, 65536 / nxt), [&](size_t z0, size_t z1) {
+            for (int iz = (int)z0; iz < (int)z1; iz++)
+                for (int ix = 0; ix < nxt; ix++) {
+                    const size_t o = (size_t)iz * pitch + ix, c = (size_t)iz * nxt + ix;
+                    L[o] = (float)(dt * lam[c]);
+                    M2[o] = (float)(2.0 * dt * mu[c]);
+                    if (iz < nzt - 1 && ix < nxt - 1) {
+                        const size_t a = (size_t)iz * (nxt - 1) + ix;
+                        MZ[o] = (float)(dt * mu_zx[a]);
+                        BXp[o] = (float)(dt * rho_xp[a]);
+                        BZp[o] = (float)(dt * rho_zp[a]);
+                    }
                 }
-            }
+        });
         FWI_TRY(d_mat.ensure(h.size() * sizeof(float)));
         CUDA_TRY(cudaMemcpyAsync(d_mat.p, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice,
                                  stream));
@@ -959,6 +961,26 @@ struct Engine {
         have_model = true;
         rb_valid = false;
         return FWI_OK;
+    }
+
+    // Raw FP64 models on the host: averaged and scaled on the device, by way of a
+    // temporary copy there (the host's average_parameters, four reciprocals per
+    // cell, where there is no room for one; the same values).
+    int set_model_lmr(const double* lam, const double* mu, const double* rho) {
+        FWI_TRY(bind());
+        const size_t n = (size_t)nzt * nxt;
+        DBuf raw;
+        if (raw.ensure(3 * n * sizeof(double)) != FWI_OK) {
+            const size_t na = (size_t)(nzt - 1) * (nxt - 1);
+            std::vector<double> mz(na), rz(na), rx(na);
+            average_parameters(nzt, nxt, mu, rho, mz.data(), rz.data(), rx.data());
+            return set_model(lam, mu, mz.data(), rz.data(), rx.data());
+        }
+        double* d = raw.as<double>();
+        const double* src[3] = {lam, mu, rho};
+        for (int k = 0; k < 3; k++)
+            CUDA_TRY(cudaMemcpyAsync(d + k * n, src[k], n * sizeof(double), cudaMemcpyHostToDevice, stream));
+        return set_model_device(d, d + n, d + 2 * n);
     }
 
     // Raw FP64 models already on the device; averages and dt scaling by a kernel.
@@ -1852,8 +1874,10 @@ struct Engine {
         FWI_TRY(grow(d_obsf, std::max<size_t>(1, (size_t)nrec) * nt * 4));
         FWI_TRY(h_stage.ensure(recs.size() * nt * 4));
         float* o = h_stage.as<float>();
-        for (size_t k = 0; k < recs.size(); k++)
-            for (int t = 0; t < nt; t++) o[k * nt + t] = (float)obs[(size_t)recs[k] * nt + t];
+        parallel_for(recs.size(), std::max<size_t>(1, 131072 / nt), [&](size_t k0, size_t k1) {
+            for (size_t k = k0; k < k1; k++)
+                for (int t = 0; t < nt; t++) o[k * nt + t] = (float)obs[(size_t)recs[k] * nt + t];
+        });
         // one copy per run of consecutive receiver indices
         size_t k = 0;
         while (k < recs.size()) {
@@ -2306,8 +2330,10 @@ struct Engine {
         stats.device_bytes = (int64_t)(allocated_bytes() + fixed_bytes());
         stats.snapshots = slots;
         if (rec_out)
-            for (size_t k = 0; k < nrows; k++)
-                for (int t = 0; t < nt; t++) rec_out[(size_t)rows[k] * nt + t] = (double)rec[k * nt + t];
+            parallel_for(nrows, std::max<size_t>(1, 131072 / nt), [&](size_t k0, size_t k1) {
+                for (size_t k = k0; k < k1; k++)
+                    for (int t = 0; t < nt; t++) rec_out[(size_t)rows[k] * nt + t] = (double)rec[k * nt + t];
+            });
         stats.h2d_bytes = last_h2d;
         stats.d2h_bytes = (int64_t)((rec_out ? nrows * nt * 4 : 0) + (obs ? nrows * 8 + 4 : 0));
         if (misfit) {
@@ -2362,6 +2388,16 @@ struct Engine {
         cudaEventDestroy(b);
         fwd_kept = false;
         return FWI_OK;
+    }
+
+    // A gradient triple from the staging buffer to the caller's FP64 arrays (at `o`).
+    void gradients_out(const float* t, size_t o, double* gl, double* gm, double* gr, double k0, double k1,
+                       double k2) const {
+        parallel_for(nf, 65536, [&](size_t i0, size_t i1) {
+            for (size_t i = i0; gl && i < i1; i++) gl[o + i] = t[i] * k0;
+            for (size_t i = i0; gm && i < i1; i++) gm[o + i] = t[nf + i] * k1;
+            for (size_t i = i0; gr && i < i1; i++) gr[o + i] = t[2 * nf + i] * k2;
+        });
     }
 
     // ---- backward --------------------------------------------------------------
@@ -2509,13 +2545,7 @@ struct Engine {
                                 : random_mode() ? (int64_t)2 * nt
                                                 : 0;
         const double k0 = out_scale(0), k1 = out_scale(1), k2 = out_scale(2);
-        for (size_t s = 0; s < ntrip && want; s++)
-            for (size_t i = 0; i < nf; i++) {
-                const float* t = g + s * 3 * nf;
-                if (gl) gl[s * nf + i] = t[i] * k0;
-                if (gm) gm[s * nf + i] = t[nf + i] * k1;
-                if (gr) gr[s * nf + i] = t[2 * nf + i] * k2;
-            }
+        for (size_t s = 0; s < ntrip && want; s++) gradients_out(g + s * 3 * nf, s * nf, gl, gm, gr, k0, k1, k2);
         bwd_done = true;
         return FWI_OK;
     }
@@ -2694,11 +2724,7 @@ struct Engine {
         CUDA_TRY(cudaStreamSynchronize(stream));
         const float* g = h_grad.as<float>();
         const double k0 = out_scale(0), k1 = out_scale(1), k2 = out_scale(2);
-        for (size_t i = 0; want && i < nf; i++) {
-            if (gl) gl[i] = g[i] * k0;
-            if (gm) gm[i] = g[nf + i] * k1;
-            if (gr) gr[i] = g[2 * nf + i] * k2;
-        }
+        if (want) gradients_out(g, 0, gl, gm, gr, k0, k1, k2);
         stats.last_forward_ms = fwd_ms;
         stats.last_backward_ms = bwd_ms;
         stats.launches = launches;
@@ -2764,19 +2790,33 @@ struct Engine {
     int storage_io(double* const f[5], bool upload) {
         FWI_TRY(bind());
         if (!d_store.p) return fail(FWI_ERR_STATE, "no FWI storage allocated");
-        std::vector<float> h((size_t)nft * 5 * nf);
-        if (!upload) CUDA_TRY(cudaMemcpy(h.data(), d_store.p, h.size() * 4, cudaMemcpyDeviceToHost));
-        for (int tf = 0; tf < nft; tf++)
-            for (int q = 0; q < 5; q++) {
-                if (!f[q]) continue;
-                float* blk = h.data() + ((size_t)tf * 5 + q) * nf;
-                double* ref = f[q] + (size_t)tf * nf;
-                for (size_t i = 0; i < nf; i++) {
-                    if (upload) blk[i] = (float)ref[i];
-                    else ref[i] = blk[i];
-                }
+        // in pieces through the page-locked staging buffer, whole time samples each
+        const size_t frame = 5 * nf, per = std::max<size_t>(1, (size_t)(4 << 20) / frame);
+        FWI_TRY(h_stage.ensure(std::min<size_t>(per, nft) * frame * 4));
+        float* h = h_stage.as<float>();
+        for (size_t t0 = 0; t0 < (size_t)nft; t0 += per) {
+            const size_t n = std::min(per, (size_t)nft - t0);
+            float* dev = d_store.as<float>() + t0 * frame;
+            if (!upload) {
+                CUDA_TRY(cudaMemcpyAsync(h, dev, n * frame * 4, cudaMemcpyDeviceToHost, stream));
+                CUDA_TRY(cudaStreamSynchronize(stream));
             }
-        if (upload) CUDA_TRY(cudaMemcpy(d_store.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice));
+            parallel_for(n * 5, std::max<size_t>(1, 131072 / nf), [&](size_t k0, size_t k1) {
+                for (size_t k = k0; k < k1; k++) {
+                    if (!f[k % 5]) continue;
+                    float* blk = h + k * nf;
+                    double* ref = f[k % 5] + (t0 + k / 5) * nf;
+                    for (size_t i = 0; i < nf; i++) {
+                        if (upload) blk[i] = (float)ref[i];
+                        else ref[i] = blk[i];
+                    }
+                }
+            });
+            if (upload) {
+                CUDA_TRY(cudaMemcpyAsync(dev, h, n * frame * 4, cudaMemcpyHostToDevice, stream));
+                CUDA_TRY(cudaStreamSynchronize(stream));
+            }
+        }
         return FWI_OK;
     }
     // CPML memory of batch slot 0 in the reference layouts, order
@@ -2987,11 +3027,7 @@ int fwi_psv_set_model(fwi_psv_engine* h, const double* lam, const double* mu, co
 int fwi_psv_set_model_lmr(fwi_psv_engine* h, const double* lam, const double* mu, const double* rho) {
     GUARD_ENGINE(h);
     if (!lam || !mu || !rho) return fail(FWI_ERR_INVALID, "null material array");
-    Engine& e = h->e;
-    const size_t na = (size_t)(e.nzt - 1) * (e.nxt - 1);
-    std::vector<double> mz(na), rz(na), rx(na);
-    fwi::average_parameters(e.nzt, e.nxt, mu, rho, mz.data(), rz.data(), rx.data());
-    return e.set_model(lam, mu, mz.data(), rz.data(), rx.data());
+    return h->e.set_model_lmr(lam, mu, rho);
 }
 
 struct fwi_psv_multi {

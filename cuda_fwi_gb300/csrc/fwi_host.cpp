@@ -9,7 +9,32 @@
 
 #include "../../include/fwi_psv.h"
 
+#include <algorithm>
+#include <system_error>
+#include <thread>
+
 namespace fwi {
+
+void parallel_for(size_t n, size_t grain, const std::function<void(size_t, size_t)>& f) {
+    size_t parts = n / std::max<size_t>(grain, 1);
+    if (parts < 2) {
+        f(0, n);
+        return;
+    }
+    static const size_t hw = std::max(1u, std::thread::hardware_concurrency());  // (reads a file)
+    parts = std::min({hw, (size_t)8, parts});
+    std::vector<std::thread> others;
+    size_t given = 0;  // pieces handed to other threads: the first ones
+    try {
+        others.reserve(parts);
+        for (; given + 1 < parts; given++)
+            others.emplace_back([&f, n, parts, given] { f(n * given / parts, n * (given + 1) / parts); });
+    } catch (const std::exception&) {
+        // no (more) threads to be had: the rest is done here
+    }
+    f(n * given / parts, n);
+    for (auto& t : others) t.join();
+}
 
 namespace {
 thread_local std::string g_last_error;

@@ -3,6 +3,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -12,6 +13,13 @@ namespace fwi {
 void set_error(const std::string& msg);
 const char* last_error();
 int fail(int status, const std::string& msg);
+
+// f(lo, hi) over pieces of [0, n), on as many host threads as pieces of at least
+// `grain` elements keep busy (at most 8, this one included); returns when all
+// are done.  For the conversions between the caller's FP64 arrays and the FP32
+// staging buffers: first touches of fresh pages and one pass of loads and
+// stores, ~1 GB/s on one thread.
+void parallel_for(size_t n, size_t grain, const std::function<void(size_t, size_t)>& f);
 
 // CUDA_week2/holbergcoeff.cu:6-60
 int holberg(int fdorder, int max_rel_err, double hc[7]);

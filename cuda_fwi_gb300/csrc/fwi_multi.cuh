@@ -61,6 +61,7 @@ struct MultiEngine {
     DBuf d_fwd, d_adj, d_ws, d_wr, d_ux, d_uz, d_grad, d_mat, d_cpml, d_srcsig, d_rec, d_resid, d_obs;
     DBuf d_rowmis, d_blow, d_snap, d_items_f, d_items_a, d_evcol, d_ev, d_evx, d_err, d_rows;
     DBuf d_mmaps, d_gids;   // TMA maps per model; member lists of the groups (events)
+    HBuf h_io;              // page-locked staging of observed data and gradients
     DBuf d_evmap;           // event maps of every model, forward then adjoint
     bool ev_map = false;    // the velocity passes of the TMA tiles inject and record
     bool mmaps_built = false;
@@ -952,13 +953,15 @@ struct MultiEngine {
         }
         // observed data (FP32, per model [nrec][nt])
         {
-            std::vector<float> h(total_rec, 0.f);
+            FWI_TRY(h_io.ensure(std::max({total_rec, total_grad, (size_t)1}) * 4));
+            float* h = h_io.as<float>();
+            std::fill(h, h + total_rec, 0.f);
             for (int b = 0; b < n; b++) {
                 const MultiItem& I = items[b];
                 if (!obs[b] && I.nrec) return fail(FWI_ERR_INVALID, "observed data of model " + std::to_string(b));
                 for (size_t i = 0; i < (size_t)I.nrec * I.nt; i++) h[I.off_rec + i] = (float)obs[b][i];
             }
-            CUDA_TRY(cudaMemcpyAsync(d_obs.p, h.data(), total_rec * 4, cudaMemcpyHostToDevice, stream));
+            CUDA_TRY(cudaMemcpyAsync(d_obs.p, h, total_rec * 4, cudaMemcpyHostToDevice, stream));
             CUDA_TRY(cudaStreamSynchronize(stream));
         }
         const bool cfree = copy_free();
@@ -1056,13 +1059,13 @@ struct MultiEngine {
         CUDA_TRY(cudaEventRecord(e1, stream));
         // results
         std::vector<double> rm(row_item.size());
-        std::vector<float> g(total_grad);
+        const float* g = h_io.as<float>();  // (the observed data have left it)
         int blow = 0;
         if (!rm.empty())
             CUDA_TRY(cudaMemcpyAsync(rm.data(), d_rowmis.p, rm.size() * 8, cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaMemcpyAsync(&blow, d_blow.p, 4, cudaMemcpyDeviceToHost, stream));
         const bool want_g = gl || gm || gr;
-        if (want_g) CUDA_TRY(cudaMemcpyAsync(g.data(), d_grad.p, total_grad * 4, cudaMemcpyDeviceToHost, stream));
+        if (want_g) CUDA_TRY(cudaMemcpyAsync(h_io.p, d_grad.p, total_grad * 4, cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
         int flag = 0;
         FWI_TRY(check_bounds_record());
@@ -1079,17 +1082,27 @@ struct MultiEngine {
             r0 += items[b].nrec;
             if (misfit) misfit[b] = s;
         }
-        for (int b = 0; b < n && want_g; b++) {
-            const MultiItem& I = items[b];
-            const size_t nf = (size_t)I.nfz * I.nfx;
-            double* outs[3] = {gl ? gl[b] : nullptr, gm ? gm[b] : nullptr, gr ? gr[b] : nullptr};
-            for (int q = 0; q < 3; q++) {
-                if (!outs[q]) continue;
-                const float* src = g.data() + I.off_grad + q * nf;
-                for (int iz = 0; iz < I.nzt; iz++)
-                    for (int ix = 0; ix < I.nxt; ix++)
-                        outs[q][(size_t)iz * I.nxt + ix] = iz < I.wz1 ? 0.0 : (double)src[(size_t)(iz - I.wz1) * I.nfx + ix];
-            }
+        if (want_g) {
+            // rows of every gradient of every model, in one go
+            std::vector<size_t> first(n + 1, 0);
+            for (int b = 0; b < n; b++) first[b + 1] = first[b] + 3 * (size_t)items[b].nzt;
+            parallel_for(first[n], 512, [&](size_t r0, size_t r1) {
+                int b = (int)(std::upper_bound(first.begin(), first.end(), r0) - first.begin()) - 1;
+                for (size_t r = r0; r < r1; r++) {
+                    while (r >= first[b + 1]) b++;
+                    const MultiItem& I = items[b];
+                    const int q = (int)((r - first[b]) / I.nzt), iz = (int)((r - first[b]) % I.nzt);
+                    double* const out[3] = {gl ? gl[b] : nullptr, gm ? gm[b] : nullptr, gr ? gr[b] : nullptr};
+                    if (!out[q]) continue;
+                    double* o = out[q] + (size_t)iz * I.nxt;
+                    if (iz < I.wz1) {
+                        std::fill(o, o + I.nxt, 0.0);
+                        continue;
+                    }
+                    const float* src = g + I.off_grad + q * (size_t)I.nfz * I.nfx + (size_t)(iz - I.wz1) * I.nfx;
+                    for (int ix = 0; ix < I.nxt; ix++) o[ix] = (double)src[ix];
+                }
+            });
         }
         stats = fwi_psv_stats{};
         stats.launches = launches_now;
