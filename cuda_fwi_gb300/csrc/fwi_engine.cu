@@ -1996,7 +1996,9 @@ struct Engine {
         CUDA_TRY(cudaMemcpy(&h, d_err.p, sizeof(int), cudaMemcpyDeviceToHost));
         if (h) {
             CUDA_TRY(cudaMemset(d_err.p, 0, sizeof(int)));
-            if (h & 16)
+            // (after a wait that ran out the later passes return at once and record
+            // nothing: non-finite values among those samples say nothing)
+            if (h == 16)
                 return fail(FWI_ERR_DIVERGED, "non-finite values in the recorded traces or the gradients "
                                               "(device watchdog); results discarded");
             return fail(FWI_ERR_CUDA, "a kernel's shared-memory pipeline wait timed out (flag " +
