@@ -91,9 +91,23 @@ struct MultiEngine {
     fwi_psv_stats stats{};
     bool tuned = false;
     std::vector<int> row_item;  // receiver rows (all items) -> item
+    // The order groups share no data, so each runs on a stream of its own within
+    // a phase (the first on `stream`): one after the other, every pass of a group
+    // ends in a wave that leaves SMs idle, which the other groups' tiles now take.
+    // Gradient of eight models of orders 4 and 8 (2.0 M + 0.5 M cells): 55.1 ms
+    // one after the other, 41.0 ms so.  Grids cut to each group's share of the
+    // SMs measured 52.6 ms (a wave cannot be filled by the other group), and a
+    // group cut in two or three streams of its own 46.2 and 49.3 ms.
+    std::vector<cudaStream_t> side;   // of groups 1..
+    std::vector<cudaEvent_t> joined;  // their last work of a phase
+    cudaEvent_t forked_at = nullptr;
+    bool forked = false;
 
     ~MultiEngine() {
         for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
+        for (cudaStream_t st : side) cudaStreamDestroy(st);
+        for (cudaEvent_t ev : joined) cudaEventDestroy(ev);
+        if (forked_at) cudaEventDestroy(forked_at);
         if (stream) cudaStreamDestroy(stream);
     }
     int bind() {
@@ -103,6 +117,35 @@ struct MultiEngine {
     void drop_graphs() {
         for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
         graphs.clear();
+    }
+    int make_side_streams() {
+        if (groups.size() < 2) return FWI_OK;
+        CUDA_TRY(cudaEventCreateWithFlags(&forked_at, cudaEventDisableTiming));
+        for (size_t g = 1; g < groups.size(); g++) {
+            side.push_back(nullptr);
+            CUDA_TRY(cudaStreamCreateWithFlags(&side.back(), cudaStreamNonBlocking));
+            joined.push_back(nullptr);
+            CUDA_TRY(cudaEventCreateWithFlags(&joined.back(), cudaEventDisableTiming));
+        }
+        return FWI_OK;
+    }
+    // Stream of group g, its work after everything queued on `stream` so far.
+    cudaStream_t group_stream(size_t g) {
+        if (!forked && !side.empty()) {
+            cudaEventRecord(forked_at, stream);
+            for (cudaStream_t st : side) cudaStreamWaitEvent(st, forked_at);
+            forked = true;
+        }
+        return g == 0 ? stream : side[g - 1];
+    }
+    // What is queued on `stream` from here on comes after every group's work.
+    void join() {
+        if (!forked) return;
+        for (size_t g = 0; g < side.size(); g++) {
+            cudaEventRecord(joined[g], side[g]);
+            cudaStreamWaitEvent(stream, joined[g]);
+        }
+        forked = false;
     }
 
     // ---- set-up ------------------------------------------------------------
@@ -334,7 +377,7 @@ struct MultiEngine {
         FWI_TRY(d_gids.ensure(gids.size() * 4));
         CUDA_TRY(cudaMemcpy(d_gids.p, gids.data(), gids.size() * 4, cudaMemcpyHostToDevice));
         for (auto& g : groups) FWI_TRY(apply_choice(*g, g->tune));
-        return FWI_OK;
+        return make_side_streams();
     }
 
     // The maps of a model's forward state held at fwd_base (+ its offset):
@@ -548,17 +591,18 @@ struct MultiEngine {
         const ItemDesc* itm = d_items_b.as<ItemDesc>() + (size_t)y * n;
         const long long msrc = (long long)(buf(x) - buf(y));
         int* err = d_err.as<int>();
-        for (auto& gp : groups) {
-            Group& g = *gp;
+        for (size_t gi = 0; gi < groups.size(); gi++) {
+            Group& g = *groups[gi];
             const int k = active(g, it);
             if (k == 0) continue;
             const int ns = g.cum_f[k];
             const dim3 gs((unsigned)std::max(1, std::min(ns, num_sms)));
-            g.tm.stress(gs, stream, mx, my, itm, g.tiles_f.as<Tile>(), ns, it, 0u, 0, msrc, err);
-            g.tm.velocity(gs, stream, mx, my, itm, g.tiles_f.as<Tile>(), ns, it, FL_INJECT, 0, msrc, err);
+            const cudaStream_t st = group_stream(gi);
+            g.tm.stress(gs, st, mx, my, itm, g.tiles_f.as<Tile>(), ns, it, 0u, 0, msrc, err);
+            g.tm.velocity(gs, st, mx, my, itm, g.tiles_f.as<Tile>(), ns, it, FL_INJECT, 0, msrc, err);
             launches_now += 2;
             if (!ev_map) {
-                events_list_kernel<<<k, 256, 0, stream>>>(itm, d_gids.as<int>() + g.gid_off, it, FL_INJECT);
+                events_list_kernel<<<k, 256, 0, st>>>(itm, d_gids.as<int>() + g.gid_off, it, FL_INJECT);
                 launches_now++;
             }
         }
@@ -598,6 +642,7 @@ struct MultiEngine {
                     break;
                 case Action::RESTORE:
                     if (a.a < 0) {
+                        join();
                         CUDA_TRY(cudaMemsetAsync(buf(wb), 0, total_state * 4, stream));
                         src = wb;
                     } else {
@@ -627,35 +672,36 @@ struct MultiEngine {
         const ItemDesc* itm = adj ? d_items_a.as<ItemDesc>() : d_items_f.as<ItemDesc>();
         const MultiMaps* mm = d_mmaps.as<MultiMaps>();
         int* err = d_err.as<int>();
-        for (auto& gp : groups) {
-            Group& g = *gp;
+        for (size_t gi = 0; gi < groups.size(); gi++) {
+            Group& g = *groups[gi];
             const int k = active(g, it);
             if (k == 0) continue;
+            const cudaStream_t st = group_stream(gi);
             const int ns = adj ? g.cum_a[k] : g.cum_f[k];
             const bool tma_s = (adj ? g.tune.amap : g.tune.fmap) == 3;
             if (tma_s) {
                 const dim3 gs((unsigned)std::max(1, std::min(ns, num_sms)));
                 const MultiMaps* ms = adj && adj_src ? adj_src : mm;
-                (adj ? g.tm.adjoint : g.tm.stress)(gs, stream, ms, ms, itm, (adj ? g.tiles_a : g.tiles_f).as<Tile>(),
+                (adj ? g.tm.adjoint : g.tm.stress)(gs, st, ms, ms, itm, (adj ? g.tiles_a : g.tiles_f).as<Tile>(),
                                                    ns, it, sflags, 0, 0, err);
             } else {
                 const int gs = std::max(1, std::min(ns, num_sms * (adj ? g.occ_a : g.occ_f)));
-                (adj ? g.ka.stress_a : g.kf.stress_f)(dim3(gs), stream, itm,
+                (adj ? g.ka.stress_a : g.kf.stress_f)(dim3(gs), st, itm,
                                                       (adj ? g.tiles_a : g.tiles_f).as<Tile>(), ns, it, sflags, err);
             }
             const int nv = g.cum_f[k];
             if (g.tune.fmap == 3) {
                 // without an event map, injection / recording of the active members in a kernel after the pass
                 const unsigned ev = vflags & (FL_INJECT | FL_RECORD);
-                g.tm.velocity(dim3((unsigned)std::max(1, std::min(nv, num_sms))), stream, mm, mm, itm,
+                g.tm.velocity(dim3((unsigned)std::max(1, std::min(nv, num_sms))), st, mm, mm, itm,
                               g.tiles_f.as<Tile>(), nv, it, vflags, adj ? 1 : 0, 0, err);
                 if (ev && !ev_map) {
-                    events_list_kernel<<<k, 256, 0, stream>>>(itm, d_gids.as<int>() + g.gid_off, it, ev);
+                    events_list_kernel<<<k, 256, 0, st>>>(itm, d_gids.as<int>() + g.gid_off, it, ev);
                     launches_now++;
                 }
             } else {
                 const int gv = std::max(1, std::min(nv, num_sms * g.occ_v));
-                g.kf.velocity(dim3(gv), stream, itm, g.tiles_f.as<Tile>(), nv, it, vflags, err);
+                g.kf.velocity(dim3(gv), st, itm, g.tiles_f.as<Tile>(), nv, it, vflags, err);
             }
             launches_now += 2;
         }
@@ -665,6 +711,7 @@ struct MultiEngine {
             step(false, it, 0u, FL_INJECT | (record ? (FL_RECORD | FL_WE) : 0u));
     }
     int state_copy(float* dst, const float* src) {
+        join();
         CUDA_TRY(device_copy(dst, src, total_state, num_sms, stream));
         return FWI_OK;
     }
@@ -673,7 +720,9 @@ struct MultiEngine {
     template <class F>
     int run_phase(const std::string& key, F&& body) {
         if (!use_graphs) {
-            FWI_TRY(body());
+            const int st = body();
+            join();
+            FWI_TRY(st);
             CUDA_TRY(cudaGetLastError());
             return FWI_OK;
         }
@@ -682,6 +731,7 @@ struct MultiEngine {
             const int64_t before = launches_now;
             CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
             const int st = body();
+            join();
             cudaGraph_t gph = nullptr;
             cudaError_t ec = cudaStreamEndCapture(stream, &gph);
             if (st != FWI_OK) {
@@ -1046,6 +1096,7 @@ struct MultiEngine {
                         FWI_TRY(state_copy(snap(a.a), d_fwd.as<float>()));
                         break;
                     case Action::RESTORE:
+                        join();
                         if (a.a < 0) CUDA_TRY(cudaMemsetAsync(d_fwd.p, 0, total_state * 4, stream));
                         else FWI_TRY(state_copy(d_fwd.as<float>(), snap(a.a)));
                         break;

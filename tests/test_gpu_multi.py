@@ -133,3 +133,25 @@ def test_forward_uses_the_gradients_mappings(tune_cache):
     assert all(t["cached"] for t in tun)
     for a, b in zip(rec_a, rec_b):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("snapshots,use_graphs", [(3, True), (3, False), (40, True)])
+def test_order_groups_side_by_side(tune_cache, snapshots, use_graphs):
+    """Three order groups of unlike length, run side by side, give what each
+    model gives in an engine of its own, bit for bit, again on a second call."""
+    specs = [dict(fdorder=4, nx=300, nz=180, nt=120, npml=12), dict(fdorder=2, nx=64, nz=36, nt=150, npml=6),
+             dict(fdorder=12, nx=70, nz=60, nt=45, npml=8), dict(fdorder=4, nx=33, nz=29, nt=80, npml=5)]
+    ps = [P.small(nrec=4, perturb=0.05, seed=90 + i, **sp) for i, sp in enumerate(specs)]
+    rng = np.random.default_rng(3)
+    obs = [1e-6 * rng.standard_normal((p.rec_x.size, p.nt)) for p in ps]
+    with MultiEngine(ps, snapshots=snapshots, use_graphs=use_graphs, autotune=False) as m:
+        recs = m.forward()
+        runs = [m.gradient(obs) for _ in range(2)]
+    for k, p in enumerate(ps):
+        with MultiEngine([p], snapshots=snapshots, use_graphs=use_graphs, autotune=False) as one:
+            assert np.array_equal(one.forward()[0], recs[k]), k
+            g1, m1 = one.gradient([obs[k]])
+        for grads, mis in runs:
+            assert mis[k] == m1[0]
+            for i in range(3):
+                assert np.array_equal(g1[0][i], grads[k][i]), (k, i)
