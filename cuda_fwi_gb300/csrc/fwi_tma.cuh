@@ -176,6 +176,16 @@ __device__ __forceinline__ void tile_coords(const TmaGrid& g, int t, int* b, int
     *z0 = FPv + (r % g.ntz) * TZ;
     *x0 = (r / g.ntz) * kTmaTX;
 }
+// A velocity pass whose states exceed L2 walks its work-list backwards: it
+// starts at the tiles that the stress pass before it left in L2 last, and so
+// does the stress pass after it.  32 shots of the 1068x568 grid (10368 tiles),
+// order 8, per launch in a chain of steps: 657 MB of DRAM traffic for the stress
+// pass and 574 MB for the velocity pass against 686 and 603 MB in the same
+// direction; the gradient of 64 such shots 372.7 -> 368.8 ms (the passes are
+// bound by more than DRAM).  Below (kL2Tiles: five fields of 129 MB) nothing is
+// gained, and six shots of 451x343 cells, order 12 (528 tiles), lost 0.6 %.
+constexpr int kL2Tiles = 3150;
+__device__ __forceinline__ int back_to_front(int t, int ntiles) { return ntiles > kL2Tiles ? ntiles - 1 - t : t; }
 
 // ---------------------------------------------------------------------------
 // two-cell arithmetic of the forward passes
@@ -981,7 +991,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     float2 hx[FP], hz[FP];
     load_weights<FP>(items, hx, hz);
     tma_pipeline<FP, G::V_STAGE>(
-        g.ntiles, err, [&](int t, int* b, int* x0, int* z0) { tile_coords(g, t, b, x0, z0, FP, kTmaTZ); },
+        g.ntiles, err,
+        [&](int t, int* b, int* x0, int* z0) { tile_coords(g, back_to_front(t, g.ntiles), b, x0, z0, FP, kTmaTZ); },
         [&](int b, int x0, int z0, float* st, uint64_t* bar) {
             velocity_issue<FP>(maps, items + b, b, x0, z0, st, bar, we);
         },
@@ -1419,7 +1430,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     tma_pipeline<FP, G::V_STAGE>(
         ntiles, err,
         [&](int t, int* b, int* x0, int* z0) {
-            const Tile T = tiles[t];
+            const Tile T = tiles[back_to_front(t, ntiles)];
             *b = T.item;
             *x0 = T.x0;
             *z0 = T.z0;
