@@ -821,6 +821,9 @@ struct Engine {
 
     ~Engine() {
         drop_graphs();
+        if (fwd_stream) cudaStreamDestroy(fwd_stream);
+        if (ev_adj) cudaEventDestroy(ev_adj);
+        for (cudaEvent_t ev : ev_read) cudaEventDestroy(ev);
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
     void drop_graphs() {
@@ -1090,6 +1093,41 @@ struct Engine {
         return b;
     }
 
+    // Recompute on a stream of its own (run_plan_ahead).
+    bool ahead = false;
+    cudaStream_t fwd_stream = nullptr;
+    cudaEvent_t ev_adj = nullptr;
+    std::vector<cudaEvent_t> ev_read;  // per state buffer: the adjoint steps that read it are done
+    // Its stream, events and second working buffer; false (the plan then runs
+    // on one stream) where the memory for them is not there.
+    bool make_ahead(int cap, int nslots) {
+        if (budget > 0 && batch_bytes(cap, nslots, strategy) + fixed_bytes() + (size_t)cap * state * 4 > budget)
+            return false;
+        const size_t before = d_fwd2.bytes, need = (size_t)cap * state * 4;
+        if (need > before) {  // (leaves as much again for what comes later)
+            size_t fr = 0, tot = 0;
+            if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || fr < 2 * need || grow(d_fwd2, need) != FWI_OK) {
+                cudaGetLastError();
+                return false;
+            }
+        }
+        if (d_fwd2.bytes != before && cudaMemsetAsync(d_fwd2.p, 0, d_fwd2.bytes, stream) != cudaSuccess) return false;
+        if (!fwd_stream && cudaStreamCreateWithFlags(&fwd_stream, cudaStreamNonBlocking) != cudaSuccess) {
+            fwd_stream = nullptr;
+            return false;
+        }
+        if (!ev_adj && cudaEventCreateWithFlags(&ev_adj, cudaEventDisableTiming) != cudaSuccess) {
+            ev_adj = nullptr;
+            return false;
+        }
+        while ((int)ev_read.size() < nslots + 2) {
+            cudaEvent_t ev = nullptr;
+            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return false;
+            ev_read.push_back(ev);
+        }
+        return true;
+    }
+
     // grow a buffer whose address is captured in graphs
     int grow(DBuf& buf, size_t n) {
         if (buf.p && n <= buf.bytes) return FWI_OK;
@@ -1244,6 +1282,7 @@ struct Engine {
         nsnap = snap_interval > 0 ? 1 + (nt - 1) / snap_interval : 0;
         if (nsnap) FWI_TRY(grow(d_snapshots, (size_t)cap * nsnap * field * 4));
         FWI_TRY(grow(d_items_a, (size_t)cap * sizeof(ItemDesc)));
+        ahead = keep && want_slots > 0 && kmap == 3 && ckpt_mode() && !exact() && !fused() && make_ahead(cap, want_slots);
         Bcap = cap;
         B = nb;
         shots.assign(ids, ids + nb);
@@ -1864,7 +1903,7 @@ struct Engine {
         return "|B" + std::to_string(B) + "|r" + std::to_string(rows.size()) + "|s" +
                std::to_string(slots) + "|st" + std::to_string(strategy) + "|t" + std::to_string(ntiles) +
                "|g" + std::to_string(grad_on ? 1 : 0) + "|m" + std::to_string(grad_mode) + "|rb" +
-               std::to_string(rb_active ? 1 : 0) + "|em" + std::to_string(ev_map ? 1 : 0) + "|fu" + std::to_string(fused() ? 1 : 0) + "|sn" +
+               std::to_string(rb_active ? 1 : 0) + "|em" + std::to_string(ev_map ? 1 : 0) + "|fu" + std::to_string(fused() ? 1 : 0) + "|ah" + std::to_string(ahead ? 1 : 0) + "|sn" +
                std::to_string(snap_interval) + "." + std::to_string(snap_field);
     }
 
@@ -2146,7 +2185,10 @@ struct Engine {
     // replayed graph.
     long long plan_recompute() const { return plan_recompute_steps(plan, nunits(), exact() && kmap != 3); }
     int state_copy(float* dst, const float* src) {
-        CUDA_TRY(device_copy(dst, src, (size_t)B * state, num_sms, stream));
+        return state_copy(dst, src, stream);
+    }
+    int state_copy(float* dst, const float* src, cudaStream_t on) {
+        CUDA_TRY(device_copy(dst, src, (size_t)B * state, num_sms, on));
         launches_now++;
         return FWI_OK;
     }
@@ -2160,27 +2202,28 @@ struct Engine {
     // State buffers with maps and descriptors of their own (step_bufs).
     bool buffered() const { return copy_free() || fused() || (kmap == 3 && exact()); }
     // Buffers a step can read or write: the checkpoint slots, d_fwd and, for
-    // the fused step, d_fwd2, for the exact adjoint d_nxt.
-    int nbufs() const { return slots + (fused() || exact() ? 2 : 1); }
+    // the fused step and the recompute running ahead, d_fwd2, for the exact adjoint d_nxt.
+    int nbufs() const { return slots + (fused() || exact() || ahead ? 2 : 1); }
     // One recompute step (stress, velocity, source injection) from the state
     // of step `it` in buffer x to the state of step it+1 in buffer y (x == y:
     // in place).  Out of place, the stress pass reads velocities and
     // stresses from x and writes the stresses to y; the velocity pass reads
     // those stresses from y and the velocities from x; CPML memories are read
     // from x and written to y.
-    void step_bufs(int x, int y, int it) {
+    void step_bufs(int x, int y, int it, cudaStream_t on = nullptr) {
+        if (!on) on = stream;
         TmaGrid gg = tgrid;
         gg.msrc = (long long)(buf(x) - buf(y));
         const ItemDesc* items = d_items_b.as<ItemDesc>() + (size_t)y * B;
-        tset.stress(dim3(grid_tma), stream, smaps_b[x], items, gg, it, 0u, d_err.as<int>());
+        tset.stress(dim3(grid_tma), on, smaps_b[x], items, gg, it, 0u, d_err.as<int>());
         VelMaps vm = vmaps_b[x];
         vm.sxx = vmaps_b[y].sxx;
         vm.szx = vmaps_b[y].szx;
         vm.szz = vmaps_b[y].szz;
-        tset.velocity(dim3(grid_tma), stream, vm, items, gg, it, FL_INJECT, d_err.as<int>());
+        tset.velocity(dim3(grid_tma), on, vm, items, gg, it, FL_INJECT, d_err.as<int>());
         launches_now += 2;
         if (!ev_map) {
-            events_kernel<<<B, 256, 0, stream>>>(items, it, FL_INJECT);
+            events_kernel<<<B, 256, 0, on>>>(items, it, FL_INJECT);
             launches_now++;
         }
     }
@@ -2561,6 +2604,7 @@ struct Engine {
     // forward fields from whichever buffer holds them.
     int run_plan_copy_free(size_t k, int last_slot, int last_state) {
         if (fused()) return run_plan_fused(k, last_slot, last_state);
+        if (ahead) return run_plan_ahead(k, last_slot, last_state);
         const int u = unit();
         std::vector<int> phys(slots);
         for (int i = 0; i < slots; i++) phys[i] = i;
@@ -2606,6 +2650,91 @@ struct Engine {
                 }
             }
         }
+        return FWI_OK;
+    }
+
+    // The same plan with the recomputed forward steps on a stream of their own:
+    // they depend on no adjoint step, so they run beside the adjoint steps of
+    // the states made before, one working buffer ahead.  A buffer is written
+    // again only after the adjoint steps that read it, an adjoint step starts
+    // after the forward steps before it in the plan.  On one stream every pass
+    // ends in a wave that leaves SMs idle and the next one starts with an empty
+    // pipeline; now the other stream's tiles run meanwhile.  Backward, order 8,
+    // one stream and two: one shot of 1068x568 cells 3.68 and 3.19 ms (80 steps),
+    // two 5.28 and 4.97, eight 16.1 and 15.8, 32 62.5 and 61.2; one shot of
+    // 2088x688 8.53 and 7.81 (100 steps), 14 48.5 and 47.2 (60 steps); three of
+    // 547x277, order 6, 10.5 and 9.2 (240 steps).  It never lost, so it is taken
+    // wherever its second working buffer fits.
+    int run_plan_ahead(size_t k, int last_slot, int last_state) {
+        const int u = unit(), nbuf = nbufs();
+        std::vector<int> phys(slots);
+        for (int i = 0; i < slots; i++) phys[i] = i;
+        int wbs[2] = {slots, slots + 1};  // the working buffers (initially d_fwd, d_fwd2)
+        int src = last_slot >= 0 ? phys[last_slot] : wbs[0];
+        // adjoint step (counted from 1) that reads the buffer and that fwd_stream has not waited for
+        std::vector<int> read_by(nbuf, 0);
+        int nadj = 0;
+        CUDA_TRY(cudaEventRecord(ev_adj, stream));
+        CUDA_TRY(cudaStreamWaitEvent(fwd_stream, ev_adj));
+        auto claim = [&](int b) -> int {  // before fwd_stream writes buffer b
+            if (read_by[b]) CUDA_TRY(cudaStreamWaitEvent(fwd_stream, ev_read[b]));
+            read_by[b] = 0;
+            return FWI_OK;
+        };
+        auto free_wb = [&]() { return read_by[wbs[0]] <= read_by[wbs[1]] ? wbs[0] : wbs[1]; };
+        auto zero = [&]() -> int {
+            src = free_wb();
+            FWI_TRY(claim(src));
+            CUDA_TRY(cudaMemsetAsync(buf(src), 0, (size_t)B * state * 4, fwd_stream));
+            return FWI_OK;
+        };
+        auto advance = [&](int t0, int t1) -> int {
+            for (int it = t0; it < t1; it++) {
+                const int dst = src == wbs[0] || src == wbs[1] ? src : free_wb();
+                FWI_TRY(claim(dst));
+                step_bufs(src, dst, it, fwd_stream);
+                src = dst;
+            }
+            return FWI_OK;
+        };
+        if (last_slot < 0) FWI_TRY(zero());
+        FWI_TRY(advance(last_state * u, (nunits() - 1) * u));
+        for (; k < plan.size(); k++) {
+            const Action& a = plan[k];
+            switch (a.kind) {
+                case Action::ADVANCE:
+                    FWI_TRY(advance(a.a * u, a.b * u));
+                    break;
+                case Action::SAVE:
+                    if (src == wbs[0] || src == wbs[1]) {
+                        int& w = src == wbs[0] ? wbs[0] : wbs[1];
+                        std::swap(phys[a.a], w);
+                        src = phys[a.a];
+                    } else {
+                        FWI_TRY(claim(phys[a.a]));
+                        FWI_TRY(state_copy(buf(phys[a.a]), buf(src), fwd_stream));
+                        src = phys[a.a];
+                    }
+                    break;
+                case Action::RESTORE:
+                    if (a.a < 0) FWI_TRY(zero());
+                    else src = phys[a.a];
+                    break;
+                case Action::ADJOINT: {
+                    const int t0 = a.a * fwi_dt, t1 = std::min(nt, (a.a + 1) * fwi_dt);
+                    CUDA_TRY(cudaEventRecord(ev_adj, fwd_stream));
+                    CUDA_TRY(cudaStreamWaitEvent(stream, ev_adj));
+                    amap_cur = &amaps_b[src];
+                    adjoint_steps(t0, t1);
+                    amap_cur = nullptr;
+                    CUDA_TRY(cudaEventRecord(ev_read[src], stream));
+                    read_by[src] = ++nadj;
+                    break;
+                }
+            }
+        }
+        CUDA_TRY(cudaEventRecord(ev_adj, fwd_stream));
+        CUDA_TRY(cudaStreamWaitEvent(stream, ev_adj));
         return FWI_OK;
     }
 
