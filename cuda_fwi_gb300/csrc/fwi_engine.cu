@@ -1120,7 +1120,7 @@ struct Engine {
             ev_adj = nullptr;
             return false;
         }
-        while ((int)ev_read.size() < nslots + 2) {
+        while ((int)ev_read.size() < nslots + 3) {
             cudaEvent_t ev = nullptr;
             if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return false;
             ev_read.push_back(ev);
@@ -1282,7 +1282,7 @@ struct Engine {
         nsnap = snap_interval > 0 ? 1 + (nt - 1) / snap_interval : 0;
         if (nsnap) FWI_TRY(grow(d_snapshots, (size_t)cap * nsnap * field * 4));
         FWI_TRY(grow(d_items_a, (size_t)cap * sizeof(ItemDesc)));
-        ahead = keep && want_slots > 0 && kmap == 3 && ckpt_mode() && !exact() && !fused() && make_ahead(cap, want_slots);
+        ahead = keep && want_slots > 0 && kmap == 3 && ckpt_mode() && !fused() && make_ahead(cap, want_slots);
         Bcap = cap;
         B = nb;
         shots.assign(ids, ids + nb);
@@ -2119,25 +2119,38 @@ struct Engine {
     // working state, `prev` state n+1.  A step goes in place when nobody else
     // needs the buffer, otherwise into a free one (there is one: at most the
     // slots, the working state and state n+1 are in use, and a state in a slot
-    // is not counted twice).
+    // is not counted twice).  With one buffer more the forward steps run ahead on
+    // a stream of their own, as in run_plan_ahead.  Backward of one shot of
+    // 868x468 cells, order 8, 120 steps: 6.16 ms on one stream, 5.45 ms on two.
     int run_plan_exact(size_t k, int last_slot, int last_state) {
         const int nbuf = nbufs();
+        const cudaStream_t fs = ahead ? fwd_stream : stream;
         std::vector<int> own(slots, -1);
         for (size_t i = 0; i < k; i++)
             if (plan[i].kind == Action::SAVE) own[plan[i].a] = plan[i].a;
         int prev = slots;  // d_fwd: the forward sweep's final state
         int cur = -1;
+        // reverse step (counted from 1) that reads the buffer and that fs has not waited for
+        std::vector<int> read_by(nbuf, 0);
+        int nadj = 0;
         auto owned = [&](int b) { return std::find(own.begin(), own.end(), b) != own.end(); };
         auto free_buffer = [&]() {
+            int best = -1;
             for (int b = nbuf - 1; b >= 0; b--)
-                if (b != prev && b != cur && !owned(b)) return b;
-            return -1;
+                if (b != prev && b != cur && !owned(b) && (best < 0 || read_by[b] < read_by[best])) best = b;
+            return best;
+        };
+        auto claim = [&](int b) -> int {  // before fs writes buffer b
+            if (read_by[b]) CUDA_TRY(cudaStreamWaitEvent(fs, ev_read[b]));
+            read_by[b] = 0;
+            return FWI_OK;
         };
         auto zero = [&]() -> int {
             cur = -1;
             const int b = free_buffer();
             if (b < 0) return fail(FWI_ERR_STATE, "no free state buffer");
-            CUDA_TRY(cudaMemsetAsync(buf(b), 0, (size_t)B * state * 4, stream));
+            FWI_TRY(claim(b));
+            CUDA_TRY(cudaMemsetAsync(buf(b), 0, (size_t)B * state * 4, fs));
             cur = b;
             return FWI_OK;
         };
@@ -2146,11 +2159,19 @@ struct Engine {
                 int dst = cur;
                 if (cur == prev || owned(cur)) dst = free_buffer();
                 if (dst < 0) return fail(FWI_ERR_STATE, "no free state buffer");
-                step_bufs(cur, dst, it);
+                FWI_TRY(claim(dst));
+                step_bufs(cur, dst, it, fs);
                 cur = dst;
             }
             return FWI_OK;
         };
+        auto order = [&](cudaStream_t after, cudaStream_t before) -> int {
+            if (!ahead) return FWI_OK;
+            CUDA_TRY(cudaEventRecord(ev_adj, before));
+            CUDA_TRY(cudaStreamWaitEvent(after, ev_adj));
+            return FWI_OK;
+        };
+        FWI_TRY(order(fs, stream));
         if (last_slot >= 0) cur = own[last_slot];
         else FWI_TRY(zero());
         FWI_TRY(advance(last_state, nt - 1));
@@ -2169,14 +2190,22 @@ struct Engine {
                     else cur = own[a.a];
                     break;
                 case Action::ADJOINT:
+                    FWI_TRY(order(stream, fs));
                     exact_launch(true, buf(cur), buf(prev), a.a, !first, true);
                     exact_launch(false, buf(cur), buf(prev), a.a, false, false);
                     first = false;
+                    if (ahead) {
+                        nadj++;
+                        for (int b : {cur, prev}) {
+                            CUDA_TRY(cudaEventRecord(ev_read[b], stream));
+                            read_by[b] = nadj;
+                        }
+                    }
                     prev = cur;
                     break;
             }
         }
-        return FWI_OK;
+        return order(stream, fs);
     }
     // Forward steps the backward runs for the plan (in units of fwi_dt): from
     // the last checkpoint of the first sweep (placed by forward()) to the last
@@ -2197,13 +2226,14 @@ struct Engine {
     // other mappings and the exact adjoint copy states in and out of slots).
     bool copy_free() const { return kmap == 3 && ckpt_mode() && !exact() && slots > 0; }
     float* buf(int k) {
-        return k < slots ? snap(k) : k == slots ? d_fwd.as<float>() : exact() ? d_nxt.as<float>() : d_fwd2.as<float>();
+        return k < slots ? snap(k) : k == slots ? d_fwd.as<float>()
+               : k == slots + 1 && exact() ? d_nxt.as<float>() : d_fwd2.as<float>();
     }
     // State buffers with maps and descriptors of their own (step_bufs).
     bool buffered() const { return copy_free() || fused() || (kmap == 3 && exact()); }
     // Buffers a step can read or write: the checkpoint slots, d_fwd and, for
     // the fused step and the recompute running ahead, d_fwd2, for the exact adjoint d_nxt.
-    int nbufs() const { return slots + (fused() || exact() || ahead ? 2 : 1); }
+    int nbufs() const { return slots + 1 + (fused() || exact() ? 1 : 0) + (ahead ? 1 : 0); }
     // One recompute step (stress, velocity, source injection) from the state
     // of step `it` in buffer x to the state of step it+1 in buffer y (x == y:
     // in place).  Out of place, the stress pass reads velocities and

@@ -32,10 +32,12 @@ def _tightest(e, snapshots, run):
     return hi
 
 
+@pytest.mark.parametrize("mode", ["reference", "exact"])
 @pytest.mark.parametrize("order,shots,slots,sample,graphs",
                          [(4, 1, 1, 1, True), (8, 1, 3, 1, False), (8, 3, 7, 1, True), (12, 2, 4, 1, True),
                           (2, 2, 5, 2, False), (6, 1, 60, 1, True)])
-def test_two_streams_agree_with_one(order, shots, slots, sample, graphs):
+def test_two_streams_agree_with_one(order, shots, slots, sample, graphs, mode):
+    sample = 1 if mode == "exact" else sample
     p = P.small(fdorder=order, nx=150, nz=60, nt=64, npml=8, nshots=shots, nrec=6, perturb=0.04, seed=21,
                 fwi=(sample, 1, 1))
     obs = np.random.default_rng(4).standard_normal((p.nrec, p.nt)) * 1e-6
@@ -44,11 +46,13 @@ def test_two_streams_agree_with_one(order, shots, slots, sample, graphs):
     for tight in (False, True):
         with Engine(p) as e:
             e.set_exec(graphs, 256, 0)  # launches per pass, not the resident loops
+            e.set_gradient_mode(mode)
             e.set_strategy("binomial", snapshots=slots)
             if tight:
                 b = _tightest(e, slots, lambda: e.forward(ids, obs, keep=True))
         with Engine(p) as e:
             e.set_exec(graphs, 256, 0)
+            e.set_gradient_mode(mode)
             e.set_strategy("binomial", snapshots=slots, budget_bytes=b if tight else 0)
             for _ in range(2):
                 rec, mis = e.forward(ids, obs, keep=True)
