@@ -420,8 +420,9 @@ def main():
         pcs = time.perf_counter() - t0
         pc.close()
         fb = [x / sub for x in algorithmic_bytes(syn, sub, fused)]  # per shot, materials shared by a launch
-        per_grad = (syn.nt + recompute) * (fb[0] + fb[1]) + syn.nt * (fb[2] + fb[3]) + \
-            syn.nt * (syn.nxt - 2 * syn.fpad) * (syn.nzt - 2 * syn.fpad) * 8  # + energy of the recording sweep
+        # (the recording sweep and the adjoint each add their energies every second
+        # step: together the one energy per step that fb[3] counts)
+        per_grad = (syn.nt + recompute) * (fb[0] + fb[1]) + syn.nt * (fb[2] + fb[3])
         bound = peak * 1e9 / per_grad
         plain.update({"scalar_cells_shot_gradients_s": 1.0 / pcs,
                       "batched_over_plain_scalar_cells": (value / world) * pcs,

@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         // sources and receivers, as after the two-pass step's velocities
         const int cv = (tid & 63) * 2 - G::HX, r = qb + (w >> 1) * 2;
         if ((flags & (FL_INJECT | FL_RECORD)) && r <= D.ez1 && r + 1 >= D.ez0 && cv >= 0 && cv < G::W)
-            pair_events(&D, x0 + cv, r, it, flags);
+            pair_events<false>(&D, x0 + cv, r, it, flags);
     }
 }
 

@@ -52,6 +52,8 @@ enum Flags : unsigned {
     FL_INJECT = 1u << 3,  // add the injection signal at source positions
     FL_RECORD = 1u << 4,  // record vz at receiver positions
     FL_REVERSE = 1u << 5, // undo a step: subtract the increments / the injection (TMA mapping)
+    FL_WE_HELD = 1u << 6, // this step's energy is left to the next one (TMA velocity pass, event map)
+    FL_WE_PAIR = 1u << 7, // with FL_WE: the step before was FL_WE_HELD
 };
 
 struct __align__(16) ItemDesc {
@@ -79,7 +81,7 @@ struct __align__(16) ItemDesc {
     float *glam, *gmu, *grho;                // [nfz][nfx]
     const float* fwd;                        // gradient source (see fwd_kind)
     const int* evmap;                        // [ez1 - ez0 + 1][pitch] what happens in a cell (EvMap)
-    long long pad1;
+    float* held;                             // as evmap: We up to a FL_WE_HELD step where it injects
 };
 
 struct Tile {

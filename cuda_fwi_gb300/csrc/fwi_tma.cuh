@@ -626,9 +626,23 @@ __device__ __forceinline__ float cell_events(const ItemDesc& D, unsigned m, floa
     }
     return v;
 }
+// Energy of two steps at once (the engine's energy_flags): a cell that injects
+// after a FL_WE_HELD step has lost that step's velocity by the next one, so its
+// sum goes on in D.held (i: its event map entry) and replaces what the
+// FL_WE_PAIR step wrote.  v: vz before the injection.  Rounded as in the pass.
+__device__ __forceinline__ void held_energy(const ItemDesc& D, unsigned m, long long i, int ix, int iz, float v,
+                                            unsigned flags) {
+    if ((m & EV_LIST) == EV_RECORD || ix < D.fpad || ix >= D.nxt - D.fpad || iz < D.fpad || iz >= D.nzt - D.fpad)
+        return;
+    const size_t c = (size_t)iz * D.pitch + ix;
+    const float vx = D.vx[c], e = __fmaf_rn(vx, vx, __fmul_rn(v, v));
+    if (flags & FL_WE_HELD) D.held[i] = __fadd_rn(D.We[c], e);
+    else D.We[c] = __fadd_rn(D.held[i], e);
+}
 // The events of a column pair in rows [r, r + kPairRows) that this thread has
 // just updated.  Not inlined: in the velocity pass's loops this code cost the whole pass 2-3 %
 // (registers), and only the warps of the rows with events come here.
+template <bool PAIRED>
 static __device__ __noinline__ void pair_events(const ItemDesc* d, int ix, int r, int it, unsigned flags) {
     const ItemDesc& D = *d;
     const int P = D.pitch;
@@ -641,6 +655,10 @@ static __device__ __noinline__ void pair_events(const ItemDesc* d, int ix, int r
         if (!inb(i + 1, (long long)(D.ez1 - D.ez0 + 1) * P, 25)) continue;
         const int2 m = __ldg(reinterpret_cast<const int2*>(D.evmap + i));
         float* vz = D.vz + (size_t)iz * P + ix;
+        if (PAIRED && (flags & (FL_WE_HELD | FL_WE_PAIR))) {
+            if (m.x) held_energy(D, (unsigned)m.x, i, ix, iz, vz[0], flags);
+            if (m.y) held_energy(D, (unsigned)m.y, i + 1, ix + 1, iz, vz[1], flags);
+        }
         if (m.x) {
             const float v = vz[0], w = cell_events(D, (unsigned)m.x, v, it, flags);
             if (w != v) vz[0] = w;
@@ -652,7 +670,7 @@ static __device__ __noinline__ void pair_events(const ItemDesc* d, int ix, int r
     }
 }
 
-template <int FP, bool INTERIOR>
+template <int FP, bool INTERIOR, bool PAIRED>
 __device__ __forceinline__ void velocity_rows(const ItemDesc& D, const float* st, int x0, int z0, unsigned flags,
                                               const float2 (&hx)[FP], const float2 (&hz)[FP], long long msrc,
                                               int lt) {
@@ -760,16 +778,21 @@ __device__ __forceinline__ void velocity_rows(const ItemDesc& D, const float* st
             }
         }
         const int ci = r * kTmaTX + cp;
-        const float2 vxn = fma2(sg, mul2(ld2(cen + ci), add2(sxx_x, szx_z)), ld2(cen + 2 * G::CEN + ci));
-        const float2 vzn = fma2(sg, mul2(ld2(cen + G::CEN + ci), add2(szx_x, szz_z)), ld2(cen + 3 * G::CEN + ci));
+        const float2 vxo = ld2(cen + 2 * G::CEN + ci), vzo = ld2(cen + 3 * G::CEN + ci);
+        const float2 vxn = fma2(sg, mul2(ld2(cen + ci), add2(sxx_x, szx_z)), vxo);
+        const float2 vzn = fma2(sg, mul2(ld2(cen + G::CEN + ci), add2(szx_x, szz_z)), vzo);
+        float2 w = make_float2(0.f, 0.f);  // We before this step's term
+        if (we) {
+            w = ld2(cen + 4 * G::CEN + ci);
+            if (PAIRED && (flags & FL_WE_PAIR)) w = add2(w, fma2(vxo, vxo, mul2(vzo, vzo)));
+        }
         if (!inb((long long)c + 1, FWI_NFIELD(D), 24)) continue;
         if constexpr (INTERIOR) {
-            if (we)
-                *reinterpret_cast<float2*>(gwe + c) = add2(ld2(cen + 4 * G::CEN + ci), fma2(vxn, vxn, mul2(vzn, vzn)));
+            if (we) *reinterpret_cast<float2*>(gwe + c) = add2(w, fma2(vxn, vxn, mul2(vzn, vzn)));
             *reinterpret_cast<float2*>(gvx + c) = vxn;
             *reinterpret_cast<float2*>(gvz + c) = vzn;
         } else {
-            if (we) st2(gwe + c, add2(ld2(cen + 4 * G::CEN + ci), fma2(vxn, vxn, mul2(vzn, vzn))), pc.on0, pc.on1);
+            if (we) st2(gwe + c, add2(w, fma2(vxn, vxn, mul2(vzn, vzn))), pc.on0, pc.on1);
             st2(gvx + c, vxn, pc.on0, pc.on1);
             st2(gvz + c, vzn, pc.on0, pc.on1);
         }
@@ -780,15 +803,17 @@ __device__ __forceinline__ void velocity_rows(const ItemDesc& D, const float* st
 // carry an event map and the flags ask for it, by the threads that own the
 // cells.  Without a map (events spread over too many rows) the engine runs
 // events_kernel after this pass: a launch of its own, 2-3 us per time step.
-template <int FP>
+// PAIRED: FL_WE_HELD and FL_WE_PAIR may be set (not in the multi-model launches,
+// which the code for them made 1.7 % slower).
+template <int FP, bool PAIRED>
 __device__ __forceinline__ void velocity_compute(const ItemDesc& D, const TmaGrid& g, const float* st, int x0,
                                                  int z0, int it, unsigned flags, const float2 (&hx)[FP],
                                                  const float2 (&hz)[FP], int lt) {
-    if (interior_warp(g, x0, z0, flags, lt)) velocity_rows<FP, true>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
-    else velocity_rows<FP, false>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
+    if (interior_warp(g, x0, z0, flags, lt)) velocity_rows<FP, true, PAIRED>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
+    else velocity_rows<FP, false, PAIRED>(D, st, x0, z0, flags, hx, hz, g.msrc, lt);
     const int wz0 = z0 + (lt >> 6) * 2;
     if ((flags & (FL_INJECT | FL_RECORD)) && wz0 <= D.ez1 && wz0 + 1 >= D.ez0)
-        pair_events(&D, x0 + (lt & (kTmaTX / 2 - 1)) * 2, wz0, it, flags);
+        pair_events<PAIRED>(&D, x0 + (lt & (kTmaTX / 2 - 1)) * 2, wz0, it, flags);
 }
 
 // Stencil weights of a launch (every slot of a launch has the same grid),
@@ -997,7 +1022,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             velocity_issue<FP>(maps, items + b, b, x0, z0, st, bar, we);
         },
         [&](int4 c, int4, const float* st, int k) {
-            velocity_compute<FP>(*reinterpret_cast<const ItemDesc*>(st + G::V_DESC), g, st, c.y, c.z, it, flags, hx,
+            velocity_compute<FP, true>(*reinterpret_cast<const ItemDesc*>(st + G::V_DESC), g, st, c.y, c.z, it, flags, hx,
                                  hz, rotated_thread(k));
         },
         g.wait_ns);
@@ -1445,7 +1470,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             staged_weights<FP>(D, hx, hz);
             TmaGrid gg = model_ranges(D);
             gg.msrc = msrc;
-            velocity_compute<FP>(D, gg, st, c.y, c.z, it, flags, hx, hz, rotated_thread(k));
+            velocity_compute<FP, false>(D, gg, st, c.y, c.z, it, flags, hx, hz, rotated_thread(k));
         });
 }
 

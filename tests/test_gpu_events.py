@@ -65,3 +65,29 @@ def test_events_over_many_rows():
             assert np.array_equal(r1[rows], rec[rows]) and m1[0] == mis[s]
             for q in range(3):
                 assert np.array_equal(g1[q][0], g[q][s])
+
+
+@pytest.mark.parametrize("order,nt", [(4, 12), (8, 13)])
+def test_energy_of_two_steps_at_once(order, nt):
+    """A large launch adds the energies of two steps at once, a launch of one of its
+    shots each step's: the same sums, in cells with sources and residuals too (the
+    last shot's sources share receivers' cells), for an odd and an even nt."""
+    n = 12
+    p = P.small(fdorder=order, nx=960, nz=500, nt=nt, npml=16, nshots=n, nrec=5, perturb=0.04, seed=7)
+    p.set_sources([300] * (n - 1) + [30, 30, 31, 44], [20] * (n - 1) + [6, 6, 6, 20],
+                  list(range(n - 1)) + [n - 1] * 4, 15.0)
+    rx = [30, 30, 31, 32, 44, 300, 301]
+    rz = [6, 6, 6, 6, 20, 20, 20]
+    p.set_receivers(np.tile(rx, n), np.tile(rz, n), np.repeat(np.arange(n, dtype=np.int32), len(rx)))
+    obs = np.random.default_rng(6).standard_normal((p.nrec, nt)) * 1e-2
+    with Engine(p) as e:
+        e.set_strategy("binomial", snapshots=4)
+        e.forward(list(range(n)), obs, keep=True)
+        e.backward()
+        all_shots = [e.energy(k) for k in (0, n - 1)]
+        for k, want in zip((0, n - 1), all_shots):
+            e.forward([k], obs, keep=True)
+            e.backward()
+            got = e.energy(0)
+            for a, b in zip(got, want):
+                assert np.count_nonzero(a) and np.array_equal(a, b)
