@@ -127,7 +127,7 @@ static void fill_event_map(int* map, int ez0, int pitch, const std::vector<int>&
 constexpr size_t kEventMapMax = 512 * 1024;
 
 // Source injection and receiver recording of one batch slot per block, after
-// a velocity pass that did neither (the TMA mapping): the injections of a
+// a velocity pass that did neither (the TMA mapping without an event map): the injections of a
 // cell are added in event order by one thread (events are sorted by column,
 // row, injections first), then the receivers read vz
 // (forward_kernel_PSV_GPU.cu:1033-1063 order).

@@ -28,7 +28,7 @@
 // before the sweep, never written there), so the stencils need no range checks.
 // Measured, 868x468 cells, order 8, us per reverse step with everything it needs
 // of the forward states: 88 as four kernels after a copy of state n and one more
-// forward step, 51 now.
+// forward step, 51 as two, 45 with the recomputed forward steps on their own stream.
 // Free surface (row fpad): the forward assigns sxx = c a_x' with
 // c = M2 (2L + M2)/(L + M2) and zeroes szx, szz there, then mirrors szx, szz of
 // rows fpad+1..2fpad onto rows fpad-1..0 with a minus sign.  The transpose

@@ -266,8 +266,8 @@ int fwi_psv_time_kernels(fwi_psv_engine* e, int reps, double ms[4]);
 /* Execution options: use_graphs != 0 captures the time loop in CUDA graphs
  * (default 1); block_x selects the thread mapping of the stencil passes:
  * 0 the default: whole time loops with the wavefields resident in shared memory
- * where the batch's grids are small enough for that to be faster (no snapshots,
- * exact gradient or random boundary), otherwise 256; 256 TMA-staged 128x16 tiles
+ * where the batch's grids are small enough for that to be faster (no snapshots or
+ * random boundary; of the exact gradient the forward sweep), otherwise 256; 256 TMA-staged 128x16 tiles
  * in persistent CTAs, one launch per pass (the same results bit for bit, except
  * that the adjoint of a stored wavefield runs on the scalar cells), 64 vectorised
  * cells (float4 per thread), 32 scalar cells, 128 (or tile_z > 0,
