@@ -759,6 +759,11 @@ struct MultiEngine {
         const char* h = std::getenv("HOME");
         return std::string(h && *h ? h : ".") + "/.cache/cuda_fwi_gb300/autotune.json";
     }
+    // (kTuneKernels: counted up when the passes change so much that choices cached
+    // for the ones before would be wrong.  2: events inside the TMA velocity pass,
+    // overlapped launches and side-by-side groups; choices of the kernels before
+    // held eight models of orders 4 and 8 at 56.7 ms a gradient, new ones give 41.0)
+    static constexpr int kTuneKernels = 2;
     std::string tune_key(const Group& g) const {
         cudaDeviceProp pr{};
         cudaGetDeviceProperties(&pr, device);
@@ -775,7 +780,7 @@ struct MultiEngine {
         for (char& c : name)
             if (c == '"' || c == '\\') c = '_';
         return name + "|sm" + std::to_string(num_sms) + "|fp" + std::to_string(g.fp) + "|cells2^" +
-               std::to_string(cb) + "|nx2^" + std::to_string(xb);
+               std::to_string(cb) + "|nx2^" + std::to_string(xb) + "|k" + std::to_string(kTuneKernels);
     }
     // The cache file: one JSON object, one entry per line, as written below.
     static std::map<std::string, TuneChoice> read_cache(const std::string& path) {
