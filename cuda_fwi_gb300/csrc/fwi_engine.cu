@@ -1446,10 +1446,14 @@ struct Engine {
     // a step of launches is ~9.5 us of launch and pipeline latency and 14 us per
     // M cells.  Measured, resident / launches: 200x200 order 4 3.1 / 9.5, order 8
     // 3.9 / 10.5, 600x380 order 8 5.7 / 13.7, order 12 9.4 / 14.6; 403x307 order 12
-    // six shots (three launches) 48 / 24; checkpointed backward of 200x200 order 4
-    // 16.4 / 28.9, 400x300 order 8 34.2 / 30.4.  A
-    // checkpointed backward adds, per adjoint step, the gradient's and ux/uz's
-    // round trips to L2 and about two saves and restores of the state.
+    // six shots (three launches) 48 / 24.  A checkpointed backward adds, per
+    // adjoint step, the gradient's and ux/uz's round trips to L2 and about two
+    // saves and restores of the state; the launches' recompute (`again` forward
+    // steps per adjoint step) runs beside their adjoint steps (run_plan_ahead).
+    // Measured, us per adjoint step with its 1.58 forward steps: 100x100 order 2
+    // 13.3 / 20.9, 200x200 order 4 15.0 / 18.3, 300x300 17.4 / 20.0, 600x400 27.6 /
+    // 29.5, order 8 400x200 22.1 / 20.5, two shots of 200x200 22.4 / 21.3 (20-cell
+    // CPML); with 2.8 forward steps 300x300 order 4 21.5 / 29.0.
     ResPlan resident_plan(int mode) const {
         ResPlan best;
         if (bx_req != 0 || tz_req != 0 || kmap != 3 || fuse || (exact() && mode != RES_FORWARD) || random_mode() ||
@@ -1461,7 +1465,7 @@ struct Engine {
         const double mcells = 1e-6 * B * (double)(nxt - 2 * fpad) * nz;
         const double again = mode == RES_BOTH ? (double)plan_recompute() / std::max(nunits(), 1) : 0.0;
         const double pass_us = 8.8 + 0.25 * fpad + 14.0 * mcells;
-        double best_us = mode == RES_BOTH ? again * pass_us + 8.0 + 22.0 * mcells : pass_us;
+        double best_us = mode == RES_BOTH ? 6.1 + 5.8 * again + 51.0 * mcells : pass_us;
         for (int k = 1; k <= std::min(B, num_sms); k++) {
             const int launches = (B + k - 1) / k;
             if (k > 1 && (B + k - 2) / (k - 1) == launches) continue;  // no fewer launches than k - 1
@@ -1476,7 +1480,7 @@ struct Engine {
                 const int groups = std::min(t.tzm, kResThreads / gw), rows_each = (t.tzm + groups - 1) / groups;
                 // (a tie goes to the smaller perimeter)
                 const double step_us = 2.2 + rows_each * kRowUs[fpad - 1] + 0.002 * (t.tzm + npm);
-                const double us = launches * (mode == RES_BOTH ? again * step_us + 2.0 + 10.5 * rows_each : step_us);
+                const double us = launches * (mode == RES_BOTH ? again * step_us - 4.1 + 2.6 * fpad + 9.5 * rows_each : step_us);
                 if (us < best_us) {
                     best_us = us;
                     best.shots = k;
