@@ -782,9 +782,22 @@ struct Engine {
     };
     ResSet rset{};
     ResPlan res_f, res_b;
-    DBuf d_inbox, d_rops_f, d_rops_b, d_revo_f, d_rev_f, d_revo_a, d_rev_a;
-    std::string rops_key_f, rops_key_b;  // what the programs on the device were made for
-    int nrops_f = 0, nrops_b = 0;
+    struct ResProgram {
+        DBuf buf;
+        std::vector<ResOp> ops;  // what buf holds
+        // Exchange tags a run uses: at most one per pass and simulation, and one per restore.
+        long long tags() const {
+            long long fwd = 0, adj = 0;
+            for (const ResOp& o : ops) {
+                if (o.kind == RES_ADV) fwd += o.b - o.a;
+                if (o.kind == RES_RESTORE) fwd++;
+                if (o.kind == RES_ADJ) adj += o.b - o.a;
+            }
+            return std::max(fwd, adj);
+        }
+    };
+    ResProgram rops_f, rops_b;
+    DBuf d_inbox, d_revo_f, d_rev_f, d_revo_a, d_rev_a;
     unsigned res_tag = 0;  // last exchange tag used
     unsigned long long wait_ns = kWaitNs;  // limit of the kernels' bounded waits
     bool stall_next = false, stall_pending = false;  // test hook: one forward step whose wait runs out
@@ -1547,24 +1560,31 @@ struct Engine {
         CUDA_TRY(cudaStreamSynchronize(stream));
         return FWI_OK;
     }
-    int resident_program(const std::vector<ResOp>& ops, DBuf& buf, int* n) {
-        FWI_TRY(buf.ensure(ops.size() * sizeof(ResOp)));
-        CUDA_TRY(cudaMemcpyAsync(buf.p, ops.data(), ops.size() * sizeof(ResOp), cudaMemcpyHostToDevice, stream));
+    // The program on the device is the one the call asks for: made anew on each call
+    // and copied when it differs from what is there (the sampling interval, the
+    // checkpoints and the plan all enter it).
+    int resident_program(std::vector<ResOp>& ops, ResProgram& pr) {
+        if (ops.size() == pr.ops.size() && std::memcmp(ops.data(), pr.ops.data(), ops.size() * sizeof(ResOp)) == 0)
+            return FWI_OK;
+        pr.ops.clear();
+        FWI_TRY(pr.buf.ensure(ops.size() * sizeof(ResOp)));
+        CUDA_TRY(cudaMemcpyAsync(pr.buf.p, ops.data(), ops.size() * sizeof(ResOp), cudaMemcpyHostToDevice, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
-        *n = (int)ops.size();
+        pr.ops.swap(ops);
         return FWI_OK;
     }
     // The program of a forward sweep (recording; saves: state, slot) or of a
-    // backward, for every shot of the batch.  `passes` bounds the exchange tags used.
-    int resident_run(const ResPlan rp, const DBuf& ops, int nops, bool backward, long long passes) {
+    // backward, for every shot of the batch.
+    int resident_run(const ResPlan rp, const ResProgram& pr, bool backward) {
+        const long long passes = pr.tags();
         const int per = rp.t.ntx * rp.t.ntz;
         const size_t words = (size_t)rset.inbox_words(rp.t.tzm);
         const size_t bytes = (size_t)rp.shots * per * 4 * words * 8, before = d_inbox.bytes;
         FWI_TRY(d_inbox.ensure(bytes));
         ResArgs a{};
         a.t = rp.t;
-        a.nops = nops;
-        a.ops = ops.as<ResOp>();
+        a.nops = (int)pr.ops.size();
+        a.ops = pr.buf.as<ResOp>();
         a.inbox = d_inbox.as<unsigned long long>();
         a.slot_stride = (long long)B * state;
         a.state = (long long)state;
@@ -1612,26 +1632,21 @@ struct Engine {
         return FWI_OK;
     }
     int resident_forward(const std::vector<std::pair<int, int>>& saves, bool store) {
-        const std::string key = "f" + shape_key() + (store ? "S" : "") + "|sv" + std::to_string(saves.size());
-        if (key != rops_key_f) {
-            std::vector<ResOp> ops;
-            const int fl = (int)(FL_WE | FL_RECORD | (store ? FL_STORE : 0u));
-            int t = 0;
-            for (const auto& sv : saves) {
-                const int ts = sv.first * unit();
-                ops.push_back({RES_ADV, t, ts, fl});
-                ops.push_back({RES_SAVE, sv.second, 0, 0});
-                t = ts;
-            }
-            ops.push_back({RES_ADV, t, nt, fl});
-            ops.push_back({RES_FINAL, 0, 0, 0});
-            rops_key_f.clear();
-            FWI_TRY(resident_program(ops, d_rops_f, &nrops_f));
-            rops_key_f = key;
+        std::vector<ResOp> ops;
+        const int fl = (int)(FL_WE | FL_RECORD | (store ? FL_STORE : 0u));
+        int t = 0;
+        for (const auto& sv : saves) {
+            const int ts = sv.first * unit();
+            ops.push_back({RES_ADV, t, ts, fl});
+            ops.push_back({RES_SAVE, sv.second, 0, 0});
+            t = ts;
         }
+        ops.push_back({RES_ADV, t, nt, fl});
+        ops.push_back({RES_FINAL, 0, 0, 0});
+        FWI_TRY(resident_program(ops, rops_f));
         CUDA_TRY(cudaMemsetAsync(d_fwd.p, 0, (size_t)B * state * 4, stream));
         CUDA_TRY(cudaMemsetAsync(d_ws.p, 0, (size_t)B * field * 4, stream));
-        FWI_TRY(resident_run(res_f, d_rops_f, nrops_f, false, (long long)nt + 1));
+        FWI_TRY(resident_run(res_f, rops_f, false));
         if (res_f.shots && !rows.empty()) {
             const int blocks = (int)std::min<size_t>((rows.size() * nt + 255) / 256, (size_t)num_sms * 4);
             watch_traces_kernel<<<std::max(blocks, 1), 256, 0, stream>>>(d_rec.as<float>(), (int)rows.size(), nt, 0, nt,
@@ -1641,43 +1656,36 @@ struct Engine {
         return FWI_OK;
     }
     int resident_backward() {
-        const std::string key = "b" + shape_key();
         const int gf = grad_on ? (int)FL_GRAD : 0;
-        if (key != rops_key_b) {
-            std::vector<ResOp> ops;
-            if (!ckpt_mode()) {
-                ops.push_back({RES_ADJ, 0, nt, gf | (int)FL_WE});
-            } else {
-                size_t k = 0;
-                int last_slot = -1, last_state = 0;
-                while (k < plan.size() && plan[k].kind != Action::ADJOINT) {
-                    if (plan[k].kind == Action::SAVE) { last_slot = plan[k].a; last_state = plan[k].b; }
-                    k++;
-                }
-                const int u = unit();
-                ops.push_back({RES_RESTORE, last_slot, 0, 0});
-                ops.push_back({RES_ADV, last_state * u, (nunits() - 1) * u, 0});
-                for (; k < plan.size(); k++) {
-                    const Action& a = plan[k];
-                    if (a.kind == Action::ADVANCE) ops.push_back({RES_ADV, a.a * u, a.b * u, 0});
-                    else if (a.kind == Action::SAVE) ops.push_back({RES_SAVE, a.a, 0, 0});
-                    else if (a.kind == Action::RESTORE) ops.push_back({RES_RESTORE, a.a, 0, 0});
-                    else ops.push_back({RES_ADJ, a.a * u, std::min(nt, (a.a + 1) * u), gf | (int)FL_WE});
-                }
+        std::vector<ResOp> ops;
+        if (!ckpt_mode()) {
+            ops.push_back({RES_ADJ, 0, nt, gf | (int)FL_WE});
+        } else {
+            size_t k = 0;
+            int last_slot = -1, last_state = 0;
+            while (k < plan.size() && plan[k].kind != Action::ADJOINT) {
+                if (plan[k].kind == Action::SAVE) { last_slot = plan[k].a; last_state = plan[k].b; }
+                k++;
             }
-            ops.push_back({RES_FINAL, 1, 0, 0});
-            rops_key_b.clear();
-            FWI_TRY(resident_program(ops, d_rops_b, &nrops_b));
-            rops_key_b = key;
+            const int u = unit();
+            ops.push_back({RES_RESTORE, last_slot, 0, 0});
+            ops.push_back({RES_ADV, last_state * u, (nunits() - 1) * u, 0});
+            for (; k < plan.size(); k++) {
+                const Action& a = plan[k];
+                if (a.kind == Action::ADVANCE) ops.push_back({RES_ADV, a.a * u, a.b * u, 0});
+                else if (a.kind == Action::SAVE) ops.push_back({RES_SAVE, a.a, 0, 0});
+                else if (a.kind == Action::RESTORE) ops.push_back({RES_RESTORE, a.a, 0, 0});
+                else ops.push_back({RES_ADJ, a.a * u, std::min(nt, (a.a + 1) * u), gf | (int)FL_WE});
+            }
         }
+        ops.push_back({RES_FINAL, 1, 0, 0});
+        FWI_TRY(resident_program(ops, rops_b));
         CUDA_TRY(cudaMemsetAsync(d_adj.p, 0, (size_t)B * state * 4, stream));
         CUDA_TRY(cudaMemsetAsync(d_wr.p, 0, (size_t)B * field * 4, stream));
         CUDA_TRY(cudaMemsetAsync(d_ux.p, 0, (size_t)B * field * 4, stream));
         CUDA_TRY(cudaMemsetAsync(d_uz.p, 0, (size_t)B * field * 4, stream));
         CUDA_TRY(cudaMemsetAsync(d_grad.p, 0, (size_t)B * 3 * nf * 4, stream));
-        // a restored state publishes its halos too
-        return resident_run(res_b, d_rops_b, nrops_b, true,
-                            (long long)nt + nrops_b + (ckpt_mode() ? plan_recompute() * unit() : 0) + 1);
+        return resident_run(res_b, rops_b, true);
     }
     // Maps of the fused step, per buffer it can read from.
     int build_fused_maps() {

@@ -90,3 +90,32 @@ def test_resident_loops_repeat_and_follow_a_changed_batch():
     for x, y in zip(first[0], again[0]):
         assert np.array_equal(x, y)
     assert np.array_equal(first[1], again[1])
+
+
+@pytest.mark.parametrize("grid,backward_resident", [((4, 200, 200, 20), True), ((8, 600, 380, 20), False)],
+                         ids=["both_sweeps", "forward_only"])
+def test_a_changed_sampling_interval_changes_the_programs(grid, backward_resident):
+    """One engine through several FWI intervals (the number of checkpoints stays, so
+    does the number of saves of the forward sweep) gives what a fresh one gives."""
+    order, nx, nz, npml = grid
+    p, obs = _case(order, nx, nz, npml, 0, 1, 120)
+
+    def run(e, interval):
+        e.set_fwi(interval, 1, 1)
+        rec, mis = e.forward([0], obs, keep=True)
+        assert e.stats()["launches"] < p.nt
+        g = e.backward()
+        assert (e.stats()["launches"] < p.nt) == backward_resident
+        return [rec, mis, *g]
+
+    def engine():
+        e = Engine(p)
+        e.set_strategy("binomial", snapshots=5)
+        return e
+
+    with engine() as e:
+        for interval in (2, 1, 3, 1, 2):
+            with engine() as fresh:
+                want = run(fresh, interval)
+            for a, b in zip(run(e, interval), want):
+                assert np.array_equal(a, b), interval
