@@ -800,7 +800,7 @@ struct Engine {
     DBuf d_inbox, d_revo_f, d_rev_f, d_revo_a, d_rev_a;
     unsigned res_tag = 0;  // last exchange tag used
     unsigned long long wait_ns = kWaitNs;  // limit of the kernels' bounded waits
-    bool stall_next = false, stall_pending = false;  // test hook: one forward step whose wait runs out
+    bool stall_next = false, stall_pending = false;  // test hook: one sweep with a wait that runs out
     bool zero_mu = false;  // some interior cell has mu == 0 (exact mode unsupported)
     // energy-weight preconditioning of each shot's gradient (fd_wave_model.cu:1004-1052)
     bool pre_on = false;
@@ -1608,6 +1608,7 @@ struct Engine {
             }
             a.tag0 = res_tag;
             res_tag += (unsigned)passes;
+            a.stall = stall_pending ? 1 : 0;
             fill_item(a.f, b, false);
             fill_item(a.a, b, true);
             a.snap = d_snap.p ? d_snap.as<float>() + (size_t)b * state : nullptr;
@@ -1627,10 +1628,13 @@ struct Engine {
                 return FWI_OK;
             }
             CUDA_TRY(ce);
+            stall_pending = false;
             launches_now++;
         }
         return FWI_OK;
     }
+    // A launch whose CTAs wait on one another (the test hook can make a wait run out).
+    static bool waits(const ResPlan& rp) { return rp.shots > 0 && rp.t.ntx * rp.t.ntz > 1; }
     int resident_forward(const std::vector<std::pair<int, int>>& saves, bool store) {
         std::vector<ResOp> ops;
         const int fl = (int)(FL_WE | FL_RECORD | (store ? FL_STORE : 0u));
@@ -2348,7 +2352,7 @@ struct Engine {
         stall_next = false;
         const std::string key = std::string("fwd") + (store ? "S" : "") + (ckpt ? "C" : "") +
                                 (obs ? "O" : "") + (stall_pending ? "X" : "") + shape_key();
-        const bool resident_loop = res_f.shots > 0 && !stall_pending;
+        const bool resident_loop = res_f.shots > 0 && (!stall_pending || waits(res_f));
         auto sweep = [&]() -> int {
             CUDA_TRY(cudaMemsetAsync(d_fwd.p, 0, (size_t)B * state * 4, stream));
             CUDA_TRY(cudaMemsetAsync(d_ws.p, 0, (size_t)B * field * 4, stream));
@@ -2519,6 +2523,10 @@ struct Engine {
         long long recompute = 0;
         CUDA_TRY(cudaEventRecord(e0, stream));
         const std::string key = std::string(ckpt_mode() ? "bwdC" : random_mode() ? "bwdR" : "bwdS") + shape_key();
+        if (waits(res_b) && stall_next) {
+            stall_pending = true;
+            stall_next = false;
+        }
         if (res_b.shots) FWI_TRY(resident_backward());
         if (!res_b.shots) FWI_TRY(run_phase(key, [&]() -> int {
             CUDA_TRY(cudaMemsetAsync(d_adj.p, 0, (size_t)B * state * 4, stream));

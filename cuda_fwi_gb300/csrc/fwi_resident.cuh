@@ -737,6 +737,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     using G = ResGeom<FP>;
     constexpr bool TWO = MODE == RES_BOTH;
     if (__syncthreads_or(*(volatile int*)A.err != 0)) return;  // an earlier launch gave up
+    if (A.stall && blockIdx.x == 0) return;
     const ItemDesc& D = A.f;
     // CPML coefficients into shared memory, fields and memories to zero
     for (int i = threadIdx.x; i < 6 * D.tp; i += kResThreads) res_smem[kResCpml + i] = D.cpml[6 * D.tp + i];

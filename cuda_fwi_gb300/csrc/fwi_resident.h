@@ -51,6 +51,7 @@ struct ResArgs {
     long long slot_stride;
     unsigned tag0;              // tags of earlier launches are <= tag0
     float one;                  // 1.0f (a multiplier the compiler cannot see)
+    int stall;                  // test hook: CTA 0 leaves at once, so its neighbours' polls run out
     int* err;
     unsigned long long wait_ns;
 };

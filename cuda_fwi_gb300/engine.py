@@ -110,11 +110,12 @@ class Engine:
         return out
 
     def set_wait_limit(self, seconds: float):
-        """Bound of every wait of the kernels on their own copies (default 2 s)."""
+        """Bound of every wait of the kernels (default 2 s)."""
         check(_capi.lib().fwi_psv_set_wait_limit(self.h, float(seconds)), "set_wait_limit")
 
     def debug_stall_next(self):
-        """Test hook: the next forward's first TMA-staged step waits for bytes that never arrive."""
+        """Test hook: the next forward's first TMA-staged step waits for bytes that never arrive; in a
+        resident time loop (forward or backward) one CTA leaves and its neighbours' waits run out."""
         check(_capi.lib().fwi_psv_debug_stall_next(self.h), "debug_stall_next")
 
     def set_stream(self, stream_handle: int | None):

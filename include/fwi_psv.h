@@ -430,8 +430,8 @@ int fwi_psv_multi_get_stats(fwi_psv_multi* m, fwi_psv_stats* out);
 /* ---- failure detection ---------------------------------------------------- */
 
 /* No counterpart in the reference (whose CUDA errors exit the process,
- * forward_kernel_PSV_GPU.cu:19-27).  Every wait of the engine's kernels on
- * their own asynchronous copies is bounded; when one runs out the kernel sets
+ * forward_kernel_PSV_GPU.cu:19-27).  Every wait of the engine's kernels, on their
+ * own asynchronous copies or (resident loops) on one another, is bounded; when one runs out the kernel sets
  * an error word, drains its copies (bounded) and returns, the later launches of
  * the call return at once, and the call returns FWI_ERR_CUDA with the engine
  * still usable.  fwi_psv_set_wait_limit sets that bound (default 2 s; 1e-6 to
@@ -442,7 +442,9 @@ int fwi_psv_set_wait_limit(fwi_psv_engine* e, double seconds);
 /* Test hook: the next forward's first TMA-staged step (the fused step, or the
  * stress pass of the two-pass step) makes one CTA expect more bytes than its
  * copies deliver, so its wait runs out and the forward returns FWI_ERR_CUDA
- * (FWI_ERR_UNSUPPORTED on the other mappings and with the exact adjoint). */
+ * (FWI_ERR_UNSUPPORTED on the other mappings and with the exact adjoint).  In a
+ * resident time loop of several tiles, of the next forward or backward, one
+ * CTA leaves at once and its neighbours' polls run out, with the same outcome. */
 int fwi_psv_debug_stall_next(fwi_psv_engine* e);
 
 /* ---- allocation-free misfit ---------------------------------------------- */

@@ -90,3 +90,36 @@ def test_nan_in_observed_data_is_caught_by_the_residual_check():
         assert ei.value.code == "FWI_ERR_DIVERGED"
         rec, mis = eng.forward([0], obs)
     assert np.isfinite(mis).all() and mis[0] > 0
+
+
+@pytest.mark.parametrize("sweep", ["forward", "backward"])
+@pytest.mark.parametrize("strategy,shots", [("binomial", 1), ("full", 3)])
+def test_resident_loop_gives_up_and_recovers(sweep, strategy, shots):
+    """The polls of the resident loops: one CTA leaves at once, its neighbours' polls
+    run out after 1 ms, the others leave on the error word; the next call is exact."""
+    p = P.small(fdorder=4, nx=200, nz=200, nt=90, npml=20, nshots=shots, nrec=7, perturb=0.04, seed=8)
+    obs = np.random.default_rng(7).standard_normal((p.nrec, p.nt)) * 1e-2
+    ids = list(range(shots))
+
+    def run(eng):
+        rec, mis = eng.forward(ids, obs, keep=True)
+        assert eng.stats()["launches"] < p.nt
+        g = eng.backward()
+        assert eng.stats()["launches"] < p.nt
+        return [rec, mis, *g]
+
+    with Engine(p) as eng:
+        eng.set_strategy(strategy, snapshots=6)
+        want = run(eng)
+    with Engine(p) as eng:
+        eng.set_strategy(strategy, snapshots=6)
+        eng.set_wait_limit(1e-3)
+        if sweep == "backward":
+            eng.forward(ids, obs, keep=True)
+        eng.debug_stall_next()
+        with pytest.raises(_capi.FwiError) as ei:
+            eng.forward(ids, obs, keep=True) if sweep == "forward" else eng.backward()
+        assert ei.value.code == "FWI_ERR_CUDA" and "timed out" in str(ei.value)
+        eng.set_wait_limit(2.0)
+        for a, b in zip(run(eng), want):
+            assert np.array_equal(a, b)
