@@ -1232,6 +1232,11 @@ struct Engine {
                     nslot_v.push_back(b);
                 }
         const size_t nrows = nrows_v.size();
+        // how the sweeps will run
+        std::vector<Action> pl;
+        if (keep && ckpt_mode()) pl = plan_binomial(nunits(), want_slots, &plan_cost);
+        const ResPlan rf = resident_plan(RES_FORWARD, nb, pl);
+        const ResPlan rb = keep ? resident_plan(ckpt_mode() ? RES_BOTH : RES_STORED, nb, pl) : ResPlan{};
         // buffers (capacity; addresses captured in graphs)
         FWI_TRY(grow(d_fwd, (size_t)cap * state * 4));
         FWI_TRY(grow(d_adj, (size_t)cap * state * 4));
@@ -1295,7 +1300,7 @@ struct Engine {
         nsnap = snap_interval > 0 ? 1 + (nt - 1) / snap_interval : 0;
         if (nsnap) FWI_TRY(grow(d_snapshots, (size_t)cap * nsnap * field * 4));
         FWI_TRY(grow(d_items_a, (size_t)cap * sizeof(ItemDesc)));
-        ahead = keep && want_slots > 0 && kmap == 3 && ckpt_mode() && !fused() && make_ahead(cap, want_slots);
+        ahead = keep && want_slots > 0 && kmap == 3 && ckpt_mode() && !fused() && !rb.shots && make_ahead(cap, want_slots);
         Bcap = cap;
         B = nb;
         shots.assign(ids, ids + nb);
@@ -1435,9 +1440,9 @@ struct Engine {
         }
         FWI_TRY(tiles_for(B));
         if (kmap == 3) FWI_TRY(build_tma_maps());
-        if (keep && ckpt_mode()) plan = plan_binomial(nunits(), slots, &plan_cost);
-        res_f = resident_plan(RES_FORWARD);
-        res_b = keep ? resident_plan(ckpt_mode() ? RES_BOTH : RES_STORED) : ResPlan{};
+        if (keep && ckpt_mode()) plan.swap(pl);
+        res_f = rf;
+        res_b = rb;
         if (res_f.shots) FWI_TRY(resident_events(res_f, slot_f, d_revo_f, d_rev_f));
         if (res_b.shots) {
             if (res_b.mode == RES_BOTH) FWI_TRY(resident_events(res_b, slot_f, d_revo_a, d_rev_a, &slot_a));
@@ -1467,7 +1472,7 @@ struct Engine {
     // 13.3 / 20.9, 200x200 order 4 15.0 / 18.3, 300x300 17.4 / 20.0, 600x400 27.6 /
     // 29.5, order 8 400x200 22.1 / 20.5, two shots of 200x200 22.4 / 21.3 (20-cell
     // CPML); with 2.8 forward steps 300x300 order 4 21.5 / 29.0.
-    ResPlan resident_plan(int mode) const {
+    ResPlan resident_plan(int mode, int nb, const std::vector<Action>& pl) const {
         ResPlan best;
         if (bx_req != 0 || tz_req != 0 || kmap != 3 || fuse || (exact() && mode != RES_FORWARD) || random_mode() ||
             snap_interval > 0 || !rset.launch)
@@ -1475,13 +1480,14 @@ struct Engine {
         static constexpr double kRowUs[kMaxHalf] = {1.2, 1.2, 1.7, 1.8, 3.3, 3.8};
         const int pairs = res_pairs(nxt, fpad), nz = nzt - 2 * fpad, most = kResTX / 2;
         const int min_rows = fsurf ? fpad + 1 : fpad;
-        const double mcells = 1e-6 * B * (double)(nxt - 2 * fpad) * nz;
-        const double again = mode == RES_BOTH ? (double)plan_recompute() / std::max(nunits(), 1) : 0.0;
+        const double mcells = 1e-6 * nb * (double)(nxt - 2 * fpad) * nz;
+        const double again =
+            mode == RES_BOTH ? (double)plan_recompute_steps(pl, nunits(), false) / std::max(nunits(), 1) : 0.0;
         const double pass_us = 8.8 + 0.25 * fpad + 14.0 * mcells;
         double best_us = mode == RES_BOTH ? 6.1 + 5.8 * again + 51.0 * mcells : pass_us;
-        for (int k = 1; k <= std::min(B, num_sms); k++) {
-            const int launches = (B + k - 1) / k;
-            if (k > 1 && (B + k - 2) / (k - 1) == launches) continue;  // no fewer launches than k - 1
+        for (int k = 1; k <= std::min(nb, num_sms); k++) {
+            const int launches = (nb + k - 1) / k;
+            if (k > 1 && (nb + k - 2) / (k - 1) == launches) continue;  // no fewer launches than k - 1
             const int tiles = num_sms / k;
             for (int ntx = (pairs + most - 1) / most; ntx <= tiles && 2 * (pairs / ntx) >= 16; ntx++) {
                 const int ntz = std::min(tiles / ntx, nz / min_rows);

@@ -137,3 +137,26 @@ def test_failing_allocator_in_the_fwi_loop():
 
 def _spent(pool):
     return pool.alloc, pool.free
+
+
+def test_second_working_buffer_only_where_the_backward_is_launched():
+    """A backward that runs as a resident loop needs no buffer for forward steps ahead of it."""
+    p = P.small(fdorder=4, nx=200, nz=200, nt=60, npml=20, nrec=6, perturb=0.04, seed=5)
+    obs = np.random.default_rng(3).standard_normal((p.nrec, p.nt)) * 1e-2
+    up = lambda v, m: -(-v // m) * m  # noqa: E731
+    pitch, tp = up(p.nxt, 32), 2 * (p.npml + 1)
+    state = 4 * up(5 * p.nzt * pitch + 4 * up(p.nzt * tp, 32) + 4 * tp * pitch, 64)
+    out, states = [], []
+    for bx in (0, 256):
+        pool = Pool()
+        A.set_device_allocator(pool.alloc, pool.free)
+        with Engine(p) as eng:
+            eng.set_strategy("binomial", snapshots=4)
+            eng.set_exec(True, bx, 0)
+            eng.forward([0], obs, keep=True)
+            out.append(eng.backward())
+            assert (eng.stats()["launches"] < p.nt) == (bx == 0)
+            states.append(sum(n == state for n in pool.live.values()))
+    assert states == [2, 3]  # forward, adjoint, and the second working buffer of the launches
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
