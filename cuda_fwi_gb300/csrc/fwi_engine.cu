@@ -1102,8 +1102,20 @@ struct Engine {
         const bool ck = strat == FWI_STORE_BINOMIAL || (strat >= 0 && exact());
         if (strat == FWI_STORE_FULL && !ck) b += (size_t)nb * nft * 5 * nf * f;
         if (ck) b += (size_t)nslots * nb * state * f;
-        if (exact()) b += (size_t)nb * (state + 9 * field) * f;  // state n+1, tmp + acc
+        if (exact()) b += (size_t)nb * (state + (3 * nf < field ? 10 : 9) * field) * f;  // state n+1, G, H (d_exh) + acc
         return b;
+    }
+    // What the budget leaves beyond batch_bytes for memory that makes a batch
+    // faster and that it can do without: the event maps, the inbox of the resident
+    // loops and the second working buffer of run_plan_ahead.
+    size_t spare = 0;
+    bool take(size_t n) {
+        if (n > spare) return false;
+        spare -= n;
+        return true;
+    }
+    size_t inbox_bytes(const ResPlan& rp) const {
+        return rp.shots ? (size_t)rp.shots * rp.t.ntx * rp.t.ntz * 4 * rset.inbox_words(rp.t.tzm) * 8 : 0;
     }
 
     // Recompute on a stream of its own (run_plan_ahead).
@@ -1114,8 +1126,6 @@ struct Engine {
     // Its stream, events and second working buffer; false (the plan then runs
     // on one stream) where the memory for them is not there.
     bool make_ahead(int cap, int nslots) {
-        if (budget > 0 && batch_bytes(cap, nslots, strategy) + fixed_bytes() + (size_t)cap * state * 4 > budget)
-            return false;
         const size_t before = d_fwd2.bytes, need = (size_t)cap * state * 4;
         if (need > before) {  // (leaves as much again for what comes later)
             size_t fr = 0, tot = 0;
@@ -1185,14 +1195,15 @@ struct Engine {
     }
     const Tile* d_tiles_p = nullptr;
 
-    int slots_for(int nb, bool keep, int* out) {
+    // extra: what the batch takes beyond batch_bytes where there is room (take).
+    int slots_for(int nb, bool keep, size_t extra, int* out) {
         *out = 0;
         if (!(keep && ckpt_mode())) return FWI_OK;
         size_t bud = budget;
         if (bud == 0) {
             size_t fr = 0, tot = 0;
             CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-            bud = (size_t)(0.9 * (double)(fr + allocated_bytes()));
+            bud = (size_t)(0.9 * (double)(fr + allocated_bytes() - (fused() ? 0 : d_fwd2.bytes)));
         }
         const int cap = std::max(Bcap, nb);
         const size_t base = batch_bytes(cap, 0, FWI_STORE_BINOMIAL) + fixed_bytes();
@@ -1205,6 +1216,9 @@ struct Engine {
                                                " checkpoints per shot");
             want = snapshots_req;
         } else {
+            // (what makes the batch faster is worth a few checkpoints, not half of them)
+            const long long less = bud > base + extra ? (long long)((bud - base - extra) / per_slot) : 0;
+            if (2 * less >= fit) fit = less;
             want = (int)std::min<long long>(fit, nunits() - 1);
         }
         *out = std::max(0, std::min(want, nunits() - 1));
@@ -1218,11 +1232,6 @@ struct Engine {
     int setup_batch(int nb, const int* ids, bool keep) {
         if (!have_model) return fail(FWI_ERR_STATE, "set a model first");
         if (nb < 1 || !ids) return fail(FWI_ERR_INVALID, "empty shot batch");
-        int want_slots = 0;
-        FWI_TRY(slots_for(nb, keep, &want_slots));
-        const int cap = std::max(Bcap, nb);
-        if (budget > 0 && batch_bytes(cap, want_slots, keep ? strategy : -1) + fixed_bytes() > budget)
-            return fail(FWI_ERR_NOMEM, "batch does not fit the memory budget");
         // receiver rows of this batch
         std::vector<int> nrows_v, nslot_v;
         for (int b = 0; b < nb; b++)
@@ -1232,11 +1241,46 @@ struct Engine {
                     nslot_v.push_back(b);
                 }
         const size_t nrows = nrows_v.size();
-        // how the sweeps will run
+        // event maps: the rows with events, the same for every slot of the batch
+        int zf[2] = {0, -1}, za[2] = {0, -1};
+        auto widen = [](int* z, int v) {
+            z[0] = z[1] < z[0] ? v : std::min(z[0], v);
+            z[1] = std::max(z[1], v);
+        };
+        for (int r : nrows_v) {
+            widen(zf, rz[r]);
+            widen(za, rz[r]);
+        }
+        for (int i = 0; i < nsrc; i++)
+            if (scomp[i] == 2 && std::find(ids, ids + nb, sshot[i]) != ids + nb) widen(zf, sz[i]);
+        const size_t map_f = (size_t)(zf[1] - zf[0] + 1) * pitch, map_a = (size_t)(za[1] - za[0] + 1) * pitch;
+        bool maps = kmap == 3 && nb * std::max(map_f, map_a) <= kEventMapMax;
+        const size_t map_bytes = maps ? nb * (map_f + map_a) * 8 : 0;  // (each with ItemDesc::held behind it)
+        // how the sweeps will run, and in what memory
         std::vector<Action> pl;
+        ResPlan rf = resident_plan(RES_FORWARD, nb, pl), rb;
+        int want_slots = 0;
+        FWI_TRY(slots_for(nb, keep, map_bytes + inbox_bytes(rf), &want_slots));
+        const int cap = std::max(Bcap, nb);
+        const size_t need = batch_bytes(cap, want_slots, keep ? strategy : -1) + fixed_bytes();
+        if (budget > 0 && need > budget) return fail(FWI_ERR_NOMEM, "batch does not fit the memory budget");
+        spare = budget > 0 ? budget - need : SIZE_MAX;
+        maps = maps && take(map_bytes);
         if (keep && ckpt_mode()) pl = plan_binomial(nunits(), want_slots, &plan_cost);
-        const ResPlan rf = resident_plan(RES_FORWARD, nb, pl);
-        const ResPlan rb = keep ? resident_plan(ckpt_mode() ? RES_BOTH : RES_STORED, nb, pl) : ResPlan{};
+        if (keep) rb = resident_plan(ckpt_mode() ? RES_BOTH : RES_STORED, nb, pl);
+        const size_t inbox = std::max(inbox_bytes(rf), inbox_bytes(rb)), inbox_before = d_inbox.bytes;
+        if (inbox && (!take(inbox) || d_inbox.ensure(inbox) != FWI_OK)) rf = rb = ResPlan{};
+        if (d_inbox.p && d_inbox.bytes != inbox_before) {
+            // tags only grow (words of earlier launches never match); fresh memory starts from zeroed words
+            CUDA_TRY(cudaMemsetAsync(d_inbox.p, 0, d_inbox.bytes, stream));
+            res_tag = 0;
+        }
+        const bool want_ahead = keep && want_slots > 0 && kmap == 3 && ckpt_mode() && !fused() && !rb.shots &&
+                                take((size_t)cap * state * 4);
+        if (keep && !want_ahead && !fused() && d_fwd2.bytes > spare) {
+            drop_graphs();
+            d_fwd2.release();
+        }
         // buffers (capacity; addresses captured in graphs)
         FWI_TRY(grow(d_fwd, (size_t)cap * state * 4));
         FWI_TRY(grow(d_adj, (size_t)cap * state * 4));
@@ -1300,7 +1344,7 @@ struct Engine {
         nsnap = snap_interval > 0 ? 1 + (nt - 1) / snap_interval : 0;
         if (nsnap) FWI_TRY(grow(d_snapshots, (size_t)cap * nsnap * field * 4));
         FWI_TRY(grow(d_items_a, (size_t)cap * sizeof(ItemDesc)));
-        ahead = keep && want_slots > 0 && kmap == 3 && ckpt_mode() && !fused() && !rb.shots && make_ahead(cap, want_slots);
+        ahead = want_ahead && make_ahead(cap, want_slots);
         Bcap = cap;
         B = nb;
         shots.assign(ids, ids + nb);
@@ -1350,19 +1394,12 @@ struct Engine {
             slot_f[b].swap(ef);
             slot_a[b].swap(ea);
         }
-        // event maps: the rows with events, the same for every slot of the batch
-        auto rows_of = [](const std::vector<int2>& ev, int* z0, int* z1) {
-            *z0 = 0;
-            *z1 = -1;
-            for (const int2& e : ev) {
-                *z0 = *z1 < *z0 ? e.x : std::min(*z0, e.x);
-                *z1 = std::max(*z1, e.x);
-            }
-        };
-        rows_of(evf, &ez0_f, &ez1_f);
-        rows_of(eva, &ez0_a, &ez1_a);
-        const size_t map_f = (size_t)(ez1_f - ez0_f + 1) * pitch, map_a = (size_t)(ez1_a - ez0_a + 1) * pitch;
-        ev_map = kmap == 3 && B * std::max(map_f, map_a) <= kEventMapMax;
+        ez0_f = zf[0];
+        ez1_f = zf[1];
+        ez0_a = za[0];
+        ez1_a = za[1];
+        ev_map = maps && d_evmap_f.ensure(std::max<size_t>(1, B * map_f) * 8) == FWI_OK &&
+                 d_evmap_a.ensure(std::max<size_t>(1, B * map_a) * 8) == FWI_OK;
         if (ev_map) {
             std::vector<int> mf(B * map_f, 0), ma(B * map_a, 0);
             for (int b = 0; b < B; b++) {
@@ -1370,8 +1407,6 @@ struct Engine {
                 fill_event_map(mf.data() + b * map_f, ez0_f, pitch, evxf, evf, cf[0], cf[nxt]);
                 fill_event_map(ma.data() + b * map_a, ez0_a, pitch, evxa, eva, ca[0], ca[nxt]);
             }
-            FWI_TRY(d_evmap_f.ensure(std::max<size_t>(1, mf.size()) * 8));  // the maps, then ItemDesc::held
-            FWI_TRY(d_evmap_a.ensure(std::max<size_t>(1, ma.size()) * 8));
             if (!mf.empty()) CUDA_TRY(cudaMemcpyAsync(d_evmap_f.p, mf.data(), mf.size() * 4, cudaMemcpyHostToDevice, stream));
             if (!ma.empty()) CUDA_TRY(cudaMemcpyAsync(d_evmap_a.p, ma.data(), ma.size() * 4, cudaMemcpyHostToDevice, stream));
         } else {
@@ -1584,9 +1619,6 @@ struct Engine {
     int resident_run(const ResPlan rp, const ResProgram& pr, bool backward) {
         const long long passes = pr.tags();
         const int per = rp.t.ntx * rp.t.ntz;
-        const size_t words = (size_t)rset.inbox_words(rp.t.tzm);
-        const size_t bytes = (size_t)rp.shots * per * 4 * words * 8, before = d_inbox.bytes;
-        FWI_TRY(d_inbox.ensure(bytes));
         ResArgs a{};
         a.t = rp.t;
         a.nops = (int)pr.ops.size();
@@ -1604,13 +1636,9 @@ struct Engine {
         a.one = 1.f;
         for (int b = 0; b < B; b += rp.shots) {
             const int n = std::min(rp.shots, B - b);
-            // tags only grow (words of earlier launches never match); fresh memory
-            // and a counter about to wrap start over from zeroed words
-            if (d_inbox.bytes != before || passes > (long long)(0xFFFFFFF0u - res_tag)) {
-                if (b == 0 || passes > (long long)(0xFFFFFFF0u - res_tag)) {
-                    CUDA_TRY(cudaMemsetAsync(d_inbox.p, 0, d_inbox.bytes, stream));
-                    res_tag = 0;
-                }
+            if (passes > (long long)(0xFFFFFFF0u - res_tag)) {  // a counter about to wrap starts over
+                CUDA_TRY(cudaMemsetAsync(d_inbox.p, 0, d_inbox.bytes, stream));
+                res_tag = 0;
             }
             a.tag0 = res_tag;
             res_tag += (unsigned)passes;
@@ -1959,7 +1987,8 @@ struct Engine {
     size_t allocated_bytes() const {
         size_t t = d_fwd.bytes + d_fwd2.bytes + d_adj.bytes + d_ws.bytes + d_wr.bytes + d_ux.bytes + d_uz.bytes +
                    d_grad.bytes + d_gsum.bytes + d_gacc.bytes + d_store.bytes + d_snap.bytes +
-                   d_rec.bytes + d_obsf.bytes + d_resid.bytes + d_nxt.bytes + d_exact.bytes;
+                   d_rec.bytes + d_obsf.bytes + d_resid.bytes + d_nxt.bytes + d_exact.bytes + d_exh.bytes +
+                   d_inbox.bytes + d_evmap_f.bytes + d_evmap_a.bytes;
         return t;
     }
 

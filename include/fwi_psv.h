@@ -185,7 +185,10 @@ int fwi_psv_set_fwi(fwi_psv_engine* e, int fwi_dt, int fwi_dx, int fwi_dz, int x
 
 /* strategy = FWI_STORE_*; snapshots = checkpoint slots per shot for
  * FWI_STORE_BINOMIAL (0 = as many as budget_bytes allows); budget_bytes = cap
- * on the engine's device memory (0 = 90% of free memory at the call). */
+ * on the engine's device memory (0 = 90% of free memory at the call); traces,
+ * residuals and observed data come on top.  Memory that only makes a batch
+ * faster (event maps, the resident loops' inbox, a second working buffer) is
+ * left out where it does not fit: the same bits, slower. */
 int fwi_psv_set_strategy(fwi_psv_engine* e, int strategy, int snapshots, size_t budget_bytes);
 
 /* Gradient formula (FWI_GRAD_*). */
