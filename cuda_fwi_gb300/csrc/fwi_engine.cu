@@ -1176,6 +1176,7 @@ struct Engine {
             FWI_TRY(grow(ts->buf, t.size() * sizeof(Tile)));
             CUDA_TRY(cudaMemcpyAsync(ts->buf.p, t.data(), t.size() * sizeof(Tile), cudaMemcpyHostToDevice,
                                      stream));
+            CUDA_TRY(cudaStreamSynchronize(stream));  // (t ends here; once per batch size)
             ts->ntiles = (int)t.size();
             ts->bx = bx;
             ts->tz = tz;
@@ -1353,6 +1354,11 @@ struct Engine {
         row_slot = nslot_v;
         fwd_kept = false;
         bwd_done = false;
+        // what is copied from here on lives until the wait at the end: a copy from
+        // pageable memory that the device can read directly may still be running when
+        // the call for it returns
+        std::vector<int> mf, ma;
+        std::vector<ItemDesc> itb;
         // events per slot, grouped by column, sorted by (z, inject-before-record, index)
         std::vector<std::vector<Ev>> slot_f(B), slot_a(B);
         std::vector<int> colf((size_t)B * (nxt + 1)), cola((size_t)B * (nxt + 1));
@@ -1401,7 +1407,8 @@ struct Engine {
         ev_map = maps && d_evmap_f.ensure(std::max<size_t>(1, B * map_f) * 8) == FWI_OK &&
                  d_evmap_a.ensure(std::max<size_t>(1, B * map_a) * 8) == FWI_OK;
         if (ev_map) {
-            std::vector<int> mf(B * map_f, 0), ma(B * map_a, 0);
+            mf.assign(B * map_f, 0);
+            ma.assign(B * map_a, 0);
             for (int b = 0; b < B; b++) {
                 const int *cf = colf.data() + (size_t)b * (nxt + 1), *ca = cola.data() + (size_t)b * (nxt + 1);
                 fill_event_map(mf.data() + b * map_f, ez0_f, pitch, evxf, evf, cf[0], cf[nxt]);
@@ -1458,7 +1465,7 @@ struct Engine {
         }
         if (buffered()) {
             const int nbuf = nbufs();
-            std::vector<ItemDesc> itb((size_t)nbuf * B);
+            itb.resize((size_t)nbuf * B);
             for (int k = 0; k < nbuf; k++)
                 for (int b = 0; b < B; b++) fill_item(itb[(size_t)k * B + b], b, false, buf(k));
             FWI_TRY(grow(d_items_b, itb.size() * sizeof(ItemDesc)));
