@@ -1048,8 +1048,8 @@ struct MultiEngine {
         // residuals and per-row misfits, one small launch per model
         CUDA_TRY(cudaMemsetAsync(d_blow.p, 0, 4, stream));
         FWI_TRY(d_rows.ensure(std::max<size_t>(1, row_item.size()) * 4));
+        std::vector<int> rr(row_item.size());  // (lives until the wait for the results)
         {
-            std::vector<int> rr(row_item.size());
             size_t r0 = 0;
             for (int b = 0; b < n; b++) {
                 for (int r = 0; r < items[b].nrec; r++) rr[r0 + r] = r;
