@@ -1514,6 +1514,15 @@ struct Engine {
     // 13.3 / 20.9, 200x200 order 4 15.0 / 18.3, 300x300 17.4 / 20.0, 600x400 27.6 /
     // 29.5, order 8 400x200 22.1 / 20.5, two shots of 200x200 22.4 / 21.3 (20-cell
     // CPML); with 2.8 forward steps 300x300 order 4 21.5 / 29.0.
+    //
+    // Over a stored wavefield the launches take their adjoint steps on the scalar
+    // cells, which round otherwise, so there the grid alone decides (a shot's
+    // gradient must not depend on how many share its call): the loop, wherever one
+    // shot's tiles fit.  Measured, us per adjoint step, resident / launches, 1, 4 and
+    // 16 shots: order 4 200x200 6.3 / 16.7, 10.7 / 20.5, 39 / 52, 700x700 20 / 29,
+    // 75 / 113, 294 / 418; order 8 200x200 7.4 / 18.4, 14.6 / 22.5, 63 / 61, 700x500
+    // 22.5 / 32.3, 88 / 93, 342 / 340; order 12 400x300 17.5 / 22.1, 48 / 47, 183 / 163,
+    // 500x400 20.6 / 23.7, 72 / 63, 285 / 249 (many shots of orders 10 and 12 lose by it).
     ResPlan resident_plan(int mode, int nb, const std::vector<Action>& pl) const {
         ResPlan best;
         if (bx_req != 0 || tz_req != 0 || kmap != 3 || fuse || (exact() && mode != RES_FORWARD) || random_mode() ||
@@ -1526,7 +1535,7 @@ struct Engine {
         const double again =
             mode == RES_BOTH ? (double)plan_recompute_steps(pl, nunits(), false) / std::max(nunits(), 1) : 0.0;
         const double pass_us = 8.8 + 0.25 * fpad + 14.0 * mcells;
-        double best_us = mode == RES_BOTH ? 6.1 + 5.8 * again + 51.0 * mcells : pass_us;
+        double best_us = mode == RES_STORED ? HUGE_VAL : mode == RES_BOTH ? 6.1 + 5.8 * again + 51.0 * mcells : pass_us;
         for (int k = 1; k <= std::min(nb, num_sms); k++) {
             const int launches = (nb + k - 1) / k;
             if (k > 1 && (nb + k - 2) / (k - 1) == launches) continue;  // no fewer launches than k - 1

@@ -188,7 +188,8 @@ int fwi_psv_set_fwi(fwi_psv_engine* e, int fwi_dt, int fwi_dx, int fwi_dz, int x
  * on the engine's device memory (0 = 90% of free memory at the call); traces,
  * residuals and observed data come on top.  Memory that only makes a batch
  * faster (event maps, the resident loops' inbox, a second working buffer) is
- * left out where it does not fit: the same bits, slower. */
+ * left out where it does not fit: the same bits, slower (but for the adjoint over
+ * a stored wavefield, whose mappings round differently: fwi_psv_set_exec). */
 int fwi_psv_set_strategy(fwi_psv_engine* e, int strategy, int snapshots, size_t budget_bytes);
 
 /* Gradient formula (FWI_GRAD_*). */
@@ -270,7 +271,9 @@ int fwi_psv_time_kernels(fwi_psv_engine* e, int reps, double ms[4]);
  * (default 1); block_x selects the thread mapping of the stencil passes:
  * 0 the default: whole time loops with the wavefields resident in shared memory
  * where the batch's grids are small enough for that to be faster (no snapshots or
- * random boundary; of the exact gradient the forward sweep), otherwise 256; 256 TMA-staged 128x16 tiles
+ * random boundary; of the exact gradient the forward sweep; the adjoint over a stored
+ * wavefield wherever one shot's grid fits, so that a shot's gradient has the same bits
+ * in every batch), otherwise 256; 256 TMA-staged 128x16 tiles
  * in persistent CTAs, one launch per pass (the same results bit for bit, except
  * that the adjoint of a stored wavefield runs on the scalar cells), 64 vectorised
  * cells (float4 per thread), 32 scalar cells, 128 (or tile_z > 0,

@@ -119,3 +119,19 @@ def test_a_changed_sampling_interval_changes_the_programs(grid, backward_residen
                 want = run(fresh, interval)
             for a, b in zip(run(e, interval), want):
                 assert np.array_equal(a, b), interval
+
+
+@pytest.mark.parametrize("grid,shots", [((8, 400, 300, 20), 8), ((6, 300, 300, 20), 16), ((12, 150, 150, 20), 24)])
+def test_stored_gradient_does_not_depend_on_the_batch(grid, shots):
+    """A shot's gradient over a stored wavefield is the same bits alone and among many."""
+    order, nx, nz, npml = grid
+    p, obs = _case(order, nx, nz, npml, 0, shots, 90)
+    with Engine(p) as e:
+        e.set_strategy("full")
+        rec, mis = e.forward(list(range(shots)), obs, keep=True)
+        g = e.backward()
+        for s in (0, shots - 1):
+            _, m1 = e.forward([s], obs, keep=True)
+            assert m1[0] == mis[s]
+            for a, b in zip(e.backward(), g):
+                assert np.count_nonzero(a[0]) and np.array_equal(a[0], b[s])
