@@ -258,6 +258,17 @@ def algorithmic_bytes(p, B, fused=False):
     return stress_fwd, vel_fwd, stress_adj, vel_adj
 
 
+def energy_bytes(p, B, block_x):
+    """Bytes per shot and time step that the energies of the recording sweep and of
+    the adjoint move beyond the 8 B per cell of algorithmic_bytes' entry 3: each
+    sweep reads and writes them every step (8 B), the TMA passes of launches of more
+    than 3150 tiles every second one (4 B; the fused step every one)."""
+    cells = (p.nxt - 2 * p.fpad) * (p.nzt - 2 * p.fpad)
+    tiles = B * -(-p.nxt // 128) * -(-(p.nzt - 2 * p.fpad) // 16)
+    pairs = block_x in (0, 256, 512) and tiles > 3150
+    return cells * ((4 if pairs and not fused_step(block_x, p.fpad) else 8) + (4 if pairs else 8) - 8)
+
+
 def main():
     args = parse()
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -420,9 +431,8 @@ def main():
         pcs = time.perf_counter() - t0
         pc.close()
         fb = [x / sub for x in algorithmic_bytes(syn, sub, fused)]  # per shot, materials shared by a launch
-        # (the recording sweep and the adjoint each add their energies every second
-        # step: together the one energy per step that fb[3] counts)
-        per_grad = (syn.nt + recompute) * (fb[0] + fb[1]) + syn.nt * (fb[2] + fb[3])
+        per_grad = (syn.nt + recompute) * (fb[0] + fb[1]) + \
+            syn.nt * (fb[2] + fb[3] + energy_bytes(syn, sub, args.block_x))
         bound = peak * 1e9 / per_grad
         plain.update({"scalar_cells_shot_gradients_s": 1.0 / pcs,
                       "batched_over_plain_scalar_cells": (value / world) * pcs,

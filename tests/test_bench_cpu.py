@@ -67,3 +67,12 @@ def test_roofline_bound_of_the_benchmark_workload():
         syn.nt * (syn.nxt - 2 * syn.fpad) * (syn.nzt - 2 * syn.fpad) * 8
     assert per_grad / 1e9 == pytest.approx(580.0, rel=0.01)
     assert 6787.6e9 / per_grad == pytest.approx(11.70, rel=0.01)
+
+
+@pytest.mark.parametrize("sub,block_x,per_cell", [(32, 0, 0), (32, 256, 0), (32, 512, 4), (9, 0, 8), (10, 0, 8), (11, 0, 0),
+                                                  (1, 256, 8), (9, 512, 8), (32, 32, 8)])
+def test_energy_bytes_of_the_sweeps(sub, block_x, per_cell):
+    """Every second step in TMA launches of more than 3150 tiles (315 a shot here), else every step."""
+    syn = P.config3(False, nshots=64)
+    cells = (syn.nxt - 2 * syn.fpad) * (syn.nzt - 2 * syn.fpad)
+    assert bench.energy_bytes(syn, sub, block_x) == per_cell * cells
