@@ -746,11 +746,11 @@ struct Engine {
     // exact discrete adjoint: forward state n+1, derivative adjoints + sensitivities, descriptors
     DBuf d_nxt, d_exact, d_exd, d_items_n, d_exh;
     ExactSet xs{};
-    // TMA mapping: kernels, tensor maps per state buffer (0 fwd, 1 adj, 2 state n+1,
-    // 3 fwd with the random-boundary materials), tile grid
+    // TMA mapping: kernels, tensor maps per state buffer (0 fwd, 1 adj, 2 fwd with
+    // the random-boundary materials), tile grid
     TmaSet tset{};
-    StressMaps smaps[4];
-    VelMaps vmaps[4];
+    StressMaps smaps[3];
+    VelMaps vmaps[3];
     AdjMaps amap;
     // Copy-free checkpointing (TMA mapping, binomial plan): buffer k < slots is
     // checkpoint memory, buffer `slots` is d_fwd; per buffer the stress and
@@ -930,7 +930,7 @@ struct Engine {
     bool random_mode() const { return strategy == FWI_STORE_RANDOM && !exact(); }
     bool state_source() const { return ckpt_mode() || random_mode(); }  // gradient reads the forward state
     // The forward sweeps run the fused step (TMA mapping, fdorder <= 8; the
-    // exact adjoint keeps its in-place two-pass steps).
+    // exact adjoint keeps the two-pass steps).
     bool fused() const { return kmap == 3 && fuse && fset.step != nullptr && !exact(); }
     int unit() const { return exact() ? 1 : fwi_dt; }
     int nunits() const { return exact() ? nt : nft; }
@@ -1811,13 +1811,12 @@ struct Engine {
         const int hx = (FPv + 3) / 4 * 4;
         const int wx = kTmaTX + 2 * hx, wz = kTmaTZ + 2 * FPv;
         const size_t rb = (size_t)pitch * 4, sb = state * 4;
-        float* bases[4] = {d_fwd.as<float>(), d_adj.as<float>(), d_nxt.p ? d_nxt.as<float>() : nullptr,
-                           rb_active ? d_fwd.as<float>() : nullptr};
-        float* webase[4] = {d_ws.as<float>(), d_wr.as<float>(), d_ws.as<float>(), d_ws.as<float>()};
-        for (int w = 0; w < 4; w++) {
+        float* bases[3] = {d_fwd.as<float>(), d_adj.as<float>(), rb_active ? d_fwd.as<float>() : nullptr};
+        float* webase[3] = {d_ws.as<float>(), d_wr.as<float>(), d_ws.as<float>()};
+        for (int w = 0; w < 3; w++) {
             float* st = bases[w];
             if (!st) continue;
-            const float* mat = w == 3 ? d_mat_rb.as<float>() : d_mat.as<float>();
+            const float* mat = w == 2 ? d_mat_rb.as<float>() : d_mat.as<float>();
             StressMaps& S = smaps[w];
             FWI_TRY(make_map(&S.vx, st + F_VX * field, nxt, nzt, Bcap, rb, sb, wx, wz));
             FWI_TRY(make_map(&S.vz, st + F_VZ * field, nxt, nzt, Bcap, rb, sb, wx, wz));
@@ -1941,7 +1940,7 @@ struct Engine {
         return FWI_OK;
     }
 
-    // Forward stress and velocity passes of one state buffer (0 fwd, 1 adj, 2 state n+1).
+    // Forward stress and velocity passes; w: tensor maps of the TMA mapping (smaps, vmaps).
     void pass_stress_fwd(int w, const ItemDesc* items, int it, unsigned flags) {
         if (kmap == 3) {
             TmaGrid g = tgrid;
@@ -2184,8 +2183,8 @@ struct Engine {
     int exact_step(int n, bool first) {
         FWI_TRY(state_copy(d_nxt.as<float>(), d_fwd.as<float>()));
         const ItemDesc* itn = d_items_n.as<ItemDesc>();
-        pass_stress_fwd(2, itn, n, 0u);
-        pass_velocity(2, itn, n, FL_INJECT);
+        pass_stress_fwd(0, itn, n, 0u);  // (these mappings go by the descriptors alone)
+        pass_velocity(0, itn, n, FL_INJECT);
         launches_now += 2;
         exact_launch(true, d_fwd.as<float>(), d_nxt.as<float>(), n, !first, true);
         exact_launch(false, d_fwd.as<float>(), d_nxt.as<float>(), n, false, false);
@@ -2303,8 +2302,8 @@ struct Engine {
         return FWI_OK;
     }
     float* snap(int slot) { return d_snap.as<float>() + (size_t)slot * B * state; }
-    // The binomial plan runs without state copies on the TMA mapping (the
-    // other mappings and the exact adjoint copy states in and out of slots).
+    // The binomial plan runs without state copies on the TMA mapping (run_plan_exact
+    // the exact adjoint's; the other mappings copy states in and out of slots).
     bool copy_free() const { return kmap == 3 && ckpt_mode() && !exact() && slots > 0; }
     float* buf(int k) {
         return k < slots ? snap(k) : k == slots ? d_fwd.as<float>()
@@ -2435,8 +2434,8 @@ struct Engine {
                 CUDA_TRY(cudaMemsetAsync(d_fwd.p, 0, (size_t)B * state * 4, stream));
                 const ItemDesc* itr = d_items_rb.as<ItemDesc>();
                 for (int it = 0; it < nt; it++) {
-                    pass_stress_fwd(3, itr, it, 0u);
-                    pass_velocity(3, itr, it, FL_INJECT);
+                    pass_stress_fwd(2, itr, it, 0u);
+                    pass_velocity(2, itr, it, FL_INJECT);
                     launches_now += 2;
                 }
             }
@@ -2522,8 +2521,8 @@ struct Engine {
             const int it = fwi_dt * (nft - 1);  // a sampled step: the gradient runs
             auto launch = [&]() {
                 // the forms of the recompute sweeps (forward) and of the adjoint
-                // sweep; source/receiver events (a separate small kernel in the
-                // TMA mapping) are left out
+                // sweep, without source/receiver events; a batch whose sweeps run as
+                // resident loops is timed on the launches it would take otherwise
                 if (k == 0 && fused()) fused_step(slots, slots + 1, it, 0u, 0u);
                 if (k == 0 && !fused()) pass_stress_fwd(0, itf, it, 0u);
                 if (k == 1) pass_velocity(0, itf, it, 0u);
@@ -2595,8 +2594,8 @@ struct Engine {
                 const ItemDesc* itr = d_items_rb.as<ItemDesc>();
                 for (int it = nt - 1; it >= 0; it--) {
                     events_kernel<<<B, 256, 0, stream>>>(itr, it, FL_INJECT | FL_REVERSE);
-                    pass_velocity(3, itr, it, FL_REVERSE);
-                    pass_stress_fwd(3, itr, it, FL_REVERSE);
+                    pass_velocity(2, itr, it, FL_REVERSE);
+                    pass_stress_fwd(2, itr, it, FL_REVERSE);
                     launches_now += 3;
                     const unsigned sf = (grad_on && it % fwi_dt == 0) ? FL_GRAD : 0u;
                     step(true, it, sf, FL_INJECT | FL_WE);
@@ -3457,9 +3456,9 @@ int fwi_psv_set_exec(fwi_psv_engine* h, int use_graphs, int block_x, int tile_z,
     e.tz_req = tile_z;
     e.batch_override = batch;
     // block_x 128 (or a tile height) selects the z-march, 32 the scalar cell
-    // mapping, 64 the vectorised cells, 256 the TMA-staged tiles, 0 the default
-    // (the TMA passes as two launches per forward step, the default), 512 the
-    // TMA mapping with the fused forward step (fdorder <= 8)
+    // mapping, 64 the vectorised cells, 256 the TMA-staged tiles as two launches per
+    // step, 0 the default (the resident loops where resident_plan takes them,
+    // otherwise as 256), 512 the TMA mapping with the fused forward step (fdorder <= 8)
     const int map = (block_x == fwi::kTileX || tile_z > 0) ? 0
                     : block_x == 32                        ? 1
                     : block_x == 256 || block_x == 512     ? 3

@@ -178,7 +178,7 @@ __device__ __forceinline__ void tile_coords(const TmaGrid& g, int t, int* b, int
 }
 // A velocity pass whose states exceed L2 walks its work-list backwards: it
 // starts at the tiles that the stress pass before it left in L2 last, and so
-// does the stress pass after it.  32 shots of the 1068x568 grid (10368 tiles),
+// does the stress pass after it.  32 shots of the 1068x568 grid (10080 tiles),
 // order 8, per launch in a chain of steps: 657 MB of DRAM traffic for the stress
 // pass and 574 MB for the velocity pass against 686 and 603 MB in the same
 // direction; the gradient of 64 such shots 372.7 -> 368.8 ms (the passes are
