@@ -263,8 +263,9 @@ int fwi_psv_checkpoint_plan(int nsteps, int slots, int* actions, int cap, int* c
  * form the checkpointed gradient runs most: ms[0] forward stress, ms[1]
  * forward velocity (no energy sum: the recompute sweeps), ms[2] adjoint stress
  * (+ux/uz and the gradient), ms[3] adjoint velocity (+energy).  Source and
- * receiver events are not included.  Needs a prior forward; it overwrites the
- * wavefield state (the retained forward is dropped). */
+ * receiver events are not included, and a batch whose sweeps run as resident
+ * loops is timed on the launches per pass it would take otherwise.  Needs a prior
+ * forward; it overwrites the wavefield state (the retained forward is dropped). */
 int fwi_psv_time_kernels(fwi_psv_engine* e, int reps, double ms[4]);
 
 /* Execution options: use_graphs != 0 captures the time loop in CUDA graphs
