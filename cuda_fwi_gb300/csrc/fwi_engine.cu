@@ -1269,8 +1269,10 @@ struct Engine {
         maps = maps && take(map_bytes);
         if (keep && ckpt_mode()) pl = plan_binomial(nunits(), want_slots, &plan_cost);
         if (keep) rb = resident_plan(ckpt_mode() ? RES_BOTH : RES_STORED, nb, pl);
+        if (!take(inbox_bytes(rf))) rf = ResPlan{};
+        if (inbox_bytes(rb) > inbox_bytes(rf) && !take(inbox_bytes(rb) - inbox_bytes(rf))) rb = ResPlan{};
         const size_t inbox = std::max(inbox_bytes(rf), inbox_bytes(rb)), inbox_before = d_inbox.bytes;
-        if (inbox && (!take(inbox) || d_inbox.ensure(inbox) != FWI_OK)) rf = rb = ResPlan{};
+        if (inbox && d_inbox.ensure(inbox) != FWI_OK) rf = rb = ResPlan{};
         if (d_inbox.p && d_inbox.bytes != inbox_before) {
             // tags only grow (words of earlier launches never match); fresh memory starts from zeroed words
             CUDA_TRY(cudaMemsetAsync(d_inbox.p, 0, d_inbox.bytes, stream));
